@@ -360,6 +360,38 @@ extern "C" void hg_destroy(hg_handle *h)
   delete h;
 }
 
+// HG_GK_* of an uploaded geometry: which kernels may leave out its zeros.
+// +0 exactly (a -0 entry would turn the signs of the products it stands in)
+// and g_ab = g_ba to the bit; anything else takes every entry.
+static bool plus_zero(double x) { return x == 0. && !std::signbit(x); }
+static bool finite_row(const double *s)
+{
+  for (int f = 0; f < 42; f++)
+    if (!std::isfinite(s[f])) return false;
+  return true;
+}
+static bool flat_geom(const double *s)
+{
+  if (!finite_row(s)) return false;
+  for (int a = 0; a < 4; a++)
+    for (int b = 0; b < 4; b++) {
+      const double e = a == b ? (a == 0 ? -1. : 1.) : 0.;
+      const double n = s[a * 4 + b], c = s[16 + a * 4 + b];
+      if (a == b ? (n != e || c != e) : !(plus_zero(n) && plus_zero(c))) return false;
+    }
+  return s[32] == 1. && s[38] == 1. && s[35] == 0. && s[36] == 0. && s[37] == 0.;
+}
+static bool axi_geom(const double *s)
+{
+  if (!finite_row(s)) return false;
+  for (int a = 0; a < 4; a++)
+    for (int b = 0; b < a; b++)
+      if (s[a * 4 + b] != s[b * 4 + a] || s[16 + a * 4 + b] != s[16 + b * 4 + a]) return false;
+  for (int f : {2, 3, 6, 8, 9, 11, 12, 14, 16 + 2, 16 + 6, 16 + 8, 16 + 9, 16 + 11, 16 + 14})
+    if (!plus_zero(s[f])) return false;
+  return s[36] == 0. && s[37] == 0. && s[38] > 0.;
+}
+
 extern "C" int hg_set_geometry(hg_handle *h, const double *geom, int64_t n_geom, const double *conn, int64_t n_conn)
 {
   if (!h || !geom) return HG_ERR_BADARG;
@@ -377,6 +409,7 @@ extern "C" int hg_set_geometry(hg_handle *h, const double *geom, int64_t n_geom,
     g.alpha = geom[34];
     for (int a = 0; a < 3; a++) g.beta[a] = geom[35 + a];
     for (int a = 0; a < 4; a++) g.ncon[a] = geom[38 + a];
+    G.gk = flat_geom(geom) ? HG_GK_FLAT : HG_GK_FULL;
   } else {
     const int N1T = h->NT[0], N2T = h->NT[1];
     if (n_geom != (int64_t)HG_NPOS * N1T * N2T || !conn || n_conn != (int64_t)G.N[0] * G.N[1]) return HG_ERR_BADARG;
@@ -388,6 +421,9 @@ extern "C" int hg_set_geometry(hg_handle *h, const double *geom, int64_t n_geom,
           const long o = ((long)pos * G.T[1] + j) * G.T[0] + i;
           for (int f = 0; f < 42; f++) t[f * G.gS + o] = s[f];
         }
+    bool axi = true;
+    for (int64_t m = 0; m < n_geom && axi; m++) axi = axi_geom(geom + 42 * m);
+    G.gk = axi ? HG_GK_AXI : HG_GK_FULL;
     HG_CK(copy_sync(h, G.geomT, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
     if (G.geomF) {  // the mixed form's FP32 face geometry
       std::vector<float> f((size_t)HG_GF * G.gS);

@@ -43,6 +43,15 @@ struct Geom {
   __host__ __device__ double det() const { return g; }
 };
 
+// What a scan of the uploaded geometry found (hg_set_geometry): FLAT is the
+// Minkowski metric in Cartesian coordinates (metric_dim 0), AXI a symmetric
+// metric_dim 2 table whose t-x2, x1-x2 and x2-x3 entries of gcov and t-x2,
+// t-x3, x1-x2 and x2-x3 entries of gcon are all +0 (Kerr-Schild in
+// COORD_DIAGONAL3).  Kernels that know the zeros leave their products out.
+#define HG_GK_FULL 0
+#define HG_GK_FLAT 1
+#define HG_GK_AXI 2
+
 // metric_dim 3 (the time-dependent metric path): the spacetime and the
 // COORD_DIAGONAL3 coordinate parameters its geometry is evaluated from.
 struct DynMetric {
@@ -80,6 +89,7 @@ struct GridDev {
   long S;            // plane size
   int NE[3];         // last physical index N+2
   int recon, flux, ct_para, bc, mdim, use_ee, cooling, rescale, nsd;
+  int gk;            // HG_GK_*: zeros and symmetry of the geometry tables, found by hg_set_geometry
   int prec;                  // HG_PREC_FP64 or HG_PREC_MIXED (FP32 face fluxes)
   // HG_PREC_MIXED only: FP32 copy of the substep's input primitives (8
   // planes of S), FP32 geometry of the faces (HG_GF planes of gS, metric_dim

@@ -23,6 +23,7 @@
 
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 #include "harmgpu.h"
 #include "hg_common.cuh"
@@ -72,6 +73,14 @@ using namespace hg;
 #ifndef HG_FLUX_MINB
 #define HG_FLUX_MINB 3
 #endif
+// the known-zero geometries hold 13 doubles of a face's geometry or none and
+// no products with its zeros: with 128 registers (4 blocks, up to 150 bytes
+// of spills) the flux of a 192x192x128 torus step takes 3.22 ms, with 168
+// 3.45, with every entry at 168 3.90; of a 128^3 flat step 1.25, 1.40, 1.61
+#ifndef HG_FLUXS_MINB
+#define HG_FLUXS_MINB 4
+#endif
+#define HG_FLUX_BLOCKS(GM) ((GM) >= HG_GM_FLAT ? HG_FLUXS_MINB : HG_FLUX_MINB)
 #ifndef HG_EE_MINB
 #define HG_EE_MINB 4
 #endif
@@ -177,16 +186,41 @@ __device__ __forceinline__ void face_prims(const GridDev &G, const double *__res
 }
 
 // ---------------------------------------------------------------------------
-// k_flux: F[d] on faces [lo, lo+n) (reference indices).
+// The face geometries the flux kernels are built for: HG_GM_CONST one struct
+// in the constant bank (metric_dim 0), HG_GM_TAB the (i, j) tables
+// (metric_dim 2), HG_GM_DYN a time level (metric_dim 3), all with every
+// entry; HG_GM_FLAT and HG_GM_AXI with the zeros of HG_GK_FLAT / HG_GK_AXI
+// left out.
+#define HG_GM_CONST 0
+#define HG_GM_TAB 2
+#define HG_GM_DYN 3
+#define HG_GM_FLAT 4
+#define HG_GM_AXI 5
+
 // HLL/LF flux of a face from its two states; writes the 8 components and
-// returns ctop.  Component by component, so no 32-value temporaries.
-__device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, const double *pr, const Geom &g, int d,
-                                            int i, int j, int k, unsigned int mult, double *__restrict__ Fd, long o)
+// returns ctop.  Component by component, so no 32-value temporaries.  The
+// normal field component is left out unless `all` is set: flux-CT replaces
+// it, and only hg_face_flux reads it.  *fin is set to whether the states are
+// finite (known-zero geometries), or to 1.
+__device__ __forceinline__ bool is_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+template <int d, class GT>
+__device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, const double *pr, const GT &g,
+                                            int i, int j, int k, unsigned int mult, double *__restrict__ Fd, long o,
+                                            int all, bool *fin)
 {
-  const int dim = d + 1;
+  constexpr int dim = d + 1;
+  constexpr bool full = std::is_same<GT, Geom>::value;
   State ql, qr;
-  if (get_state(pl, g, G.gam, ql)) book_face(G, i, j, k, mult);
-  if (get_state(pr, g, G.gam, qr)) book_face(G, i, j, k, mult);
+  const int badl = get_state(pl, g, G.gam, ql), badr = get_state(pr, g, G.gam, qr);
+  if (full) {
+    if (badl) book_face(G, i, j, k, mult);
+    if (badr) book_face(G, i, j, k, mult);
+    *fin = true;
+  } else {
+    // ucon[0] and bsq are infinite or NaN if any of ucon, bcon is
+    *fin = !(badl | badr) && is_finite((ql.ucon[0] + ql.bsq) + (qr.ucon[0] + qr.bsq));
+  }
   double cmaxl, cminl, cmaxr, cminr;
   vchar_fast(ql, g, dim, G.gam, &cmaxl, &cminl);
   vchar_fast(qr, g, dim, G.gam, &cmaxr, &cminr);
@@ -195,11 +229,12 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
   const double a1 = 0. > -cminl ? 0. : -cminl;
   const double cmin = fabs(a1 > -cminr ? a1 : -cminr);
   const double ctop = cmin > cmax ? cmin : cmax;
-  const double gg = g.g;
+  const double gg = g.det();
   if (G.flux == 1) {
     const double den = cmax + cmin + HG_SMALL;
 #pragma unroll
     for (int l = 0; l < HG_NPR; l++) {
+      if (l == B1 + d && !(full && all)) continue;
       const double Ul = flux_comp(pl, ql, 0, gg, l), Ur = flux_comp(pr, qr, 0, gg, l);
       const double Fl = flux_comp(pl, ql, dim, gg, l), Fr = flux_comp(pr, qr, dim, gg, l);
       Fd[l * G.S + o] = (cmax * Fl + cmin * Fr - cmax * cmin * (Ur - Ul)) / den;
@@ -207,6 +242,7 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
   } else {
 #pragma unroll
     for (int l = 0; l < HG_NPR; l++) {
+      if (l == B1 + d && !(full && all)) continue;
       const double Ul = flux_comp(pl, ql, 0, gg, l), Ur = flux_comp(pr, qr, 0, gg, l);
       const double Fl = flux_comp(pl, ql, dim, gg, l), Fr = flux_comp(pr, qr, dim, gg, l);
       Fd[l * G.S + o] = 0.5 * (Fl + Fr - ctop * (Ur - Ul));
@@ -215,12 +251,55 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
   return ctop;
 }
 
+// The same face with every entry of the geometry: states that are not finite
+// (or whose gamma fails) under a known-zero geometry, where 0 * inf matters.
+// sl, sr: the states, one value every ls doubles.
+template <int d>
+__device__ __noinline__ double face_flux_full(const GridDev &G, const double *sl, const double *sr, int ls, int i,
+                                              int j, int k, unsigned int mult, long o)
+{
+  double pl[HG_NPR], pr[HG_NPR];
+  for (int l = 0; l < HG_NPR; l++) {
+    pl[l] = sl[l * ls];
+    pr[l] = sr[l * ls];
+  }
+  Geom g;
+  load_geom(G, d, i, j, g, k, 0);  // metric_dim 0 or 2: no time levels
+  bool fin;
+  return face_flux<d>(G, pl, pr, g, i, j, k, mult, G.F[d], o, 0, &fin);
+}
+
+// One face of geometry GM; sl, sr as in face_flux_full.
+template <int GM, int d>
+__device__ __forceinline__ double flux_at(const GridDev &G, const double *pl, const double *pr, int i, int j, int k,
+                                          unsigned int mult, long o, int slot, int all, bool *fin)
+{
+  if (GM == HG_GM_FLAT) return face_flux<d>(G, pl, pr, GeomFlat(), i, j, k, mult, G.F[d], o, 0, fin);
+  if (GM == HG_GM_AXI) {
+    GeomAxi g;
+    load_face_geom<d>(G, i, j, g);
+    return face_flux<d>(G, pl, pr, g, i, j, k, mult, G.F[d], o, 0, fin);
+  }
+  if (GM == HG_GM_CONST) return face_flux<d>(G, pl, pr, G.g0, i, j, k, mult, G.F[d], o, all, fin);
+  Geom g;
+  load_geom(G, d, i, j, g, k, slot);  // metric_dim 3: time level `slot`
+  return face_flux<d>(G, pl, pr, g, i, j, k, mult, G.F[d], o, all, fin);
+}
+
+// fix_flux(), bounds.c:2263-2275: no mass inflow through r_in, r_out
+__device__ __forceinline__ void fix_flux(const GridDev &G, int i, long o)
+{
+  double *fr = G.F[0] + RHO * G.S + o;
+  if (i == HG_NGH && *fr > 0) *fr = 0.;
+  if (i == G.NE[0] + 1 && *fr < 0) *fr = 0.;
+}
+
 // ---------------------------------------------------------------------------
 // k_flux: F[d] on faces [lo, lo+n) (reference indices), one thread per face.
-template <bool RS, int MDIM, int d>
-__global__ void __launch_bounds__(HG_BLK, HG_FLUX_MINB) k_flux(const __grid_constant__ GridDev G, const double *__restrict__ ph,
+template <bool RS, int GM, int d>
+__global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux(const __grid_constant__ GridDev G, const double *__restrict__ ph,
                                                  int lo0, int lo1, int lo2, int n0, int n1, int n2, unsigned int mult,
-                                                 int slot)
+                                                 int slot, int all)
 {
   const unsigned total = (unsigned)n0 * n1 * n2;  // < 2^31 (hg_init)
   double vmax = 0.;
@@ -231,20 +310,18 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_MINB) k_flux(const __grid_cons
     const int k = lo2 + (int)(tq / (unsigned)n1);
     double pl[HG_NPR], pr[HG_NPR];
     face_prims<RS>(G, ph, d, i, j, k, pl, pr);
-    double ctop;
     const long o = off3(G, i, j, k);
-    if (MDIM == 0) {
-      ctop = face_flux(G, pl, pr, G.g0, d, i, j, k, mult, G.F[d], o);
-    } else {
-      Geom g;
-      load_geom(G, d, i, j, g, k, slot);
-      ctop = face_flux(G, pl, pr, g, d, i, j, k, mult, G.F[d], o);
+    bool fin;
+    double ctop = flux_at<GM, d>(G, pl, pr, i, j, k, mult, o, slot, all, &fin);
+    if (GM >= HG_GM_FLAT && !fin) {
+      double sl[HG_NPR], sr[HG_NPR];  // copies, so that pl and pr stay in registers
+      for (int l = 0; l < HG_NPR; l++) {
+        sl[l] = pl[l];
+        sr[l] = pr[l];
+      }
+      ctop = face_flux_full<d>(G, sl, sr, 1, i, j, k, mult, o);
     }
-    if (d == 0 && G.bc == 10) {  // fix_flux(), bounds.c:2263-2275: no mass inflow through r_in, r_out
-      double *fr = G.F[0] + RHO * G.S + o;
-      if (i == HG_NGH && *fr > 0) *fr = 0.;
-      if (i == G.NE[0] + 1 && *fr < 0) *fr = 0.;
-    }
+    if (d == 0 && G.bc == 10) fix_flux(G, i, o);
     if (i >= HG_NGH && i <= G.NE[0] && j >= HG_NGH && j <= G.NE[1] && k >= HG_NGH && k <= G.NE[2])
       if (ctop > vmax) vmax = ctop;
   }
@@ -322,11 +399,11 @@ __device__ __forceinline__ void strip_recon(const GridDev &G, const double *__re
   }
 }
 
-template <bool RS, int MDIM, int d, int NF>
-__global__ void __launch_bounds__(HG_BLK, HG_FLUX_MINB) k_flux_strip(const __grid_constant__ GridDev G,
+template <bool RS, int GM, int d, int NF>
+__global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux_strip(const __grid_constant__ GridDev G,
                                                                    const double *__restrict__ ph, int lo0, int lo1,
                                                                    int lo2, int n0, int n1, int n2, unsigned int mult,
-                                                                   int slot)
+                                                                   int slot, int all)
 {
   extern __shared__ double sm[];  // 16 * NF * HG_BLK doubles: the strip's face states
   const int tx = threadIdx.x;
@@ -368,19 +445,11 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_MINB) k_flux_strip(const __gri
         pr[l] = sm[(2 * NF * l + NF + s) * HG_BLK + tx];
       }
       const long o = o0 + s * st;
-      double ctop;
-      if (MDIM == 0) {
-        ctop = face_flux(G, pl, pr, G.g0, d, i, j, k, mult, G.F[d], o);
-      } else {
-        Geom g;
-        load_geom(G, d, i, j, g, k, slot);  // metric_dim 3: time level `slot`
-        ctop = face_flux(G, pl, pr, g, d, i, j, k, mult, G.F[d], o);
-      }
-      if (d == 0 && G.bc == 10) {  // fix_flux(), bounds.c:2263-2275: no mass inflow through r_in, r_out
-        double *fr = G.F[0] + RHO * G.S + o;
-        if (i == HG_NGH && *fr > 0) *fr = 0.;
-        if (i == G.NE[0] + 1 && *fr < 0) *fr = 0.;
-      }
+      bool fin;
+      double ctop = flux_at<GM, d>(G, pl, pr, i, j, k, mult, o, slot, all, &fin);
+      if (GM >= HG_GM_FLAT && !fin)
+        ctop = face_flux_full<d>(G, sm + s * HG_BLK + tx, sm + (NF + s) * HG_BLK + tx, 2 * NF * HG_BLK, i, j, k, mult, o);
+      if (d == 0 && G.bc == 10) fix_flux(G, i, o);
       if (i >= HG_NGH && i <= G.NE[0] && j >= HG_NGH && j <= G.NE[1] && k >= HG_NGH && k <= G.NE[2])
         if (ctop > vmax) vmax = ctop;
     }
@@ -1416,11 +1485,11 @@ static inline void mark(EventRec *r, int cls, cudaStream_t s)
 // torus NF = 2 measured best, and hg_autotune chooses per grid.
 template <bool RS, int MDIM, int d, int NF>
 static void launch_strip_nf(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, const int *lo,
-                            const int *n, unsigned int mult, int slot)
+                            const int *n, unsigned int mult, int slot, int all)
 {
   const size_t smem = sizeof(double) * 16 * NF * HG_BLK;
   k_flux_strip<RS, MDIM, d, NF>
-      <<<L.grid_flux, HG_BLK, smem, s>>>(G, ph, lo[0], lo[1], lo[2], n[0], n[1], n[2], mult, slot);
+      <<<L.grid_flux, HG_BLK, smem, s>>>(G, ph, lo[0], lo[1], lo[2], n[0], n[1], n[2], mult, slot, all);
 }
 
 template <bool RS, int MDIM, int d, int NF>
@@ -1460,8 +1529,11 @@ int fallback_blocks_per_sm(bool rs)
 // stream capture: called by hg_init.
 cudaError_t prepare_kernels()
 {
-  const cudaError_t r[6] = {strip_attrs_rm<false, 0>(), strip_attrs_rm<true, 0>(), strip_attrs_rm<false, 2>(),
-                            strip_attrs_rm<true, 2>(),  strip_attrs_rm<false, 3>(), strip_attrs_rm<true, 3>()};
+  const cudaError_t r[9] = {strip_attrs_rm<false, HG_GM_CONST>(), strip_attrs_rm<true, HG_GM_CONST>(),
+                            strip_attrs_rm<false, HG_GM_TAB>(),   strip_attrs_rm<true, HG_GM_TAB>(),
+                            strip_attrs_rm<false, HG_GM_DYN>(),   strip_attrs_rm<true, HG_GM_DYN>(),
+                            strip_attrs_rm<false, HG_GM_FLAT>(),  strip_attrs_rm<false, HG_GM_AXI>(),
+                            strip_attrs_rm<true, HG_GM_AXI>()};
   for (cudaError_t x : r)
     if (x != cudaSuccess) return x;
   return cudaSuccess;
@@ -1470,15 +1542,15 @@ cudaError_t prepare_kernels()
 // strips of L.strip_nf faces (1, 2 or 3: a launch-configuration choice)
 template <bool RS, int MDIM, int d>
 static void launch_strip(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, const int *lo,
-                         const int *n, unsigned int mult, int slot)
+                         const int *n, unsigned int mult, int slot, int all)
 {
-  if (L.strip_nf <= 1) launch_strip_nf<RS, MDIM, d, 1>(G, L, s, ph, lo, n, mult, slot);
-  else if (L.strip_nf == 2) launch_strip_nf<RS, MDIM, d, 2>(G, L, s, ph, lo, n, mult, slot);
-  else launch_strip_nf<RS, MDIM, d, 3>(G, L, s, ph, lo, n, mult, slot);
+  if (L.strip_nf <= 1) launch_strip_nf<RS, MDIM, d, 1>(G, L, s, ph, lo, n, mult, slot, all);
+  else if (L.strip_nf == 2) launch_strip_nf<RS, MDIM, d, 2>(G, L, s, ph, lo, n, mult, slot, all);
+  else launch_strip_nf<RS, MDIM, d, 3>(G, L, s, ph, lo, n, mult, slot, all);
 }
 
 static void launch_flux_dir(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, int d,
-                            EventRec *R, int slot)
+                            EventRec *R, int slot, int all)
 {
     int lo[3], n[3];
     unsigned int mult = 1;
@@ -1504,22 +1576,30 @@ static void launch_flux_dir(const GridDev &G, const LaunchCfg &L, cudaStream_t s
       return;
     }
 #define HG_FLUX(RSV, MD, DD) \
-  k_flux<RSV, MD, DD><<<L.grid_flux, HG_BLK, 0, s>>>(G, ph, lo[0], lo[1], lo[2], n[0], n[1], n[2], mult, slot)
+  k_flux<RSV, MD, DD><<<L.grid_flux, HG_BLK, 0, s>>>(G, ph, lo[0], lo[1], lo[2], n[0], n[1], n[2], mult, slot, \
+                                                all)
 #define HG_STRIP(RSV, MD, DD) \
-  launch_strip<RSV, MD, DD>(G, L, s, ph, lo, n, mult, slot)
+  launch_strip<RSV, MD, DD>(G, L, s, ph, lo, n, mult, slot, all)
 #define HG_FLUX_D(RSV, MD) \
   if (d == 0) { if (G.deg[0] || !L.strip_x1) HG_FLUX(RSV, MD, 0); else HG_STRIP(RSV, MD, 0); } \
   else if (d == 1) { if (G.deg[1]) HG_FLUX(RSV, MD, 1); else HG_STRIP(RSV, MD, 1); } \
   else { if (G.deg[2]) HG_FLUX(RSV, MD, 2); else HG_STRIP(RSV, MD, 2); }
+    // hg_face_flux (all) takes every entry of the geometry, so that the
+    // signs of its zeros are the reference's too
+    const int gk = all ? HG_GK_FULL : G.gk;
     if (G.mdim == 0) {
-      if (G.rescale) { HG_FLUX_D(true, 0) }
-      else { HG_FLUX_D(false, 0) }
+      if (G.rescale) { HG_FLUX_D(true, HG_GM_CONST) }
+      else if (gk == HG_GK_FLAT) { HG_FLUX_D(false, HG_GM_FLAT) }
+      else { HG_FLUX_D(false, HG_GM_CONST) }
     } else if (G.mdim == 3) {  // geometry of time level `slot`
-      if (G.rescale) { HG_FLUX_D(true, 3) }
-      else { HG_FLUX_D(false, 3) }
+      if (G.rescale) { HG_FLUX_D(true, HG_GM_DYN) }
+      else { HG_FLUX_D(false, HG_GM_DYN) }
+    } else if (gk == HG_GK_AXI) {
+      if (G.rescale) { HG_FLUX_D(true, HG_GM_AXI) }
+      else { HG_FLUX_D(false, HG_GM_AXI) }
     } else {
-      if (G.rescale) { HG_FLUX_D(true, 2) }
-      else { HG_FLUX_D(false, 2) }
+      if (G.rescale) { HG_FLUX_D(true, HG_GM_TAB) }
+      else { HG_FLUX_D(false, HG_GM_TAB) }
     }
 #undef HG_FLUX_D
 #undef HG_STRIP
@@ -1540,7 +1620,7 @@ static void launch_substep(const GridDev &G, const LaunchCfg &L, cudaStream_t s,
     k_conn_dyn<<<L.grid_upd, HG_BLK, 0, s>>>(G, sub, 0.5 * sub);
   }
   // (the mixed form's FP32 copy of ph is already current: put_state)
-  for (int d = 0; d < 3; d++) launch_flux_dir(G, L, s, ph, d, R, sub);
+  for (int d = 0; d < 3; d++) launch_flux_dir(G, L, s, ph, d, R, sub, 0);
   {
     int lo[3], n[3];
     for (int a = 0; a < 3; a++) {
@@ -1716,7 +1796,7 @@ void launch_face_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int 
 {
   k_reset_max<<<1, 1, 0, s>>>(G.sc, d + 1);
   if (G.prec == HG_PREC_MIXED) launch_to_f32(G, L.grid_upd, s, G.p);
-  launch_flux_dir(G, L, s, G.p, d, nullptr, 0);
+  launch_flux_dir(G, L, s, G.p, d, nullptr, 0, 1);
 }
 
 void launch_fixup_bounds(const GridDev &G, const LaunchCfg &L, cudaStream_t s)

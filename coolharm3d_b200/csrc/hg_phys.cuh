@@ -98,12 +98,65 @@ __device__ __forceinline__ void load_geom(const GridDev &G, int pos, int i, int 
   g.ncon[3] = __ldg(t + 41 * s);
 }
 
+// Geometries whose zeros are known at compile time (HG_GK_FLAT, HG_GK_AXI),
+// for the face fluxes: the overloads below leave out the products with a
+// zero entry.  For finite states a sum without its +-0 terms is the same
+// number (only the sign of a zero result can differ), so face_flux checks
+// that the states are finite and the sums that consume its fluxes
+// (update_zone, k_emf) start from or add +0, which takes the sign back.
+struct GeomFlat {
+  __device__ double con(int a, int b) const { return a == b ? (a == 0 ? -1. : 1.) : 0.; }
+  __device__ double det() const { return 1.; }
+};
+struct GeomAxi {
+  double c00, c01, c03, c11, c13, c22, c33;  // gcov
+  double n00, n0d, ndd;                      // gcon of the face's direction d
+  double nc0, b0, g;                         // ncon[0], beta[0], sqrt(-g)
+  __device__ double con(int a, int b) const { return a == 0 ? (b == 0 ? n00 : n0d) : ndd; }
+  __device__ double det() const { return g; }
+};
+template <int d>
+__device__ __forceinline__ void load_face_geom(const GridDev &G, int i, int j, GeomAxi &g)
+{
+  const double *t = G.geomT + ((long)d * G.T[1] + j) * G.T[0] + i;  // metric_dim 2: x1, x2 are resolved
+  const long s = G.gS;
+  g.c00 = __ldg(t + 16 * s);
+  g.c01 = __ldg(t + 17 * s);
+  g.c03 = __ldg(t + 19 * s);
+  g.c11 = __ldg(t + 21 * s);
+  g.c13 = __ldg(t + 23 * s);
+  g.c22 = __ldg(t + 26 * s);
+  g.c33 = __ldg(t + 31 * s);
+  g.n00 = __ldg(t);
+  g.n0d = d == 0 ? __ldg(t + s) : 0.;
+  g.ndd = __ldg(t + 5 * (d + 1) * s);
+  g.g = __ldg(t + 32 * s);
+  g.b0 = __ldg(t + 35 * s);
+  g.nc0 = __ldg(t + 38 * s);
+}
+
 template <class T, class GT>
 __device__ __forceinline__ void lower4(const T *v, const GT &g, T *w)  // metric.c:338
 {
 #pragma unroll
   for (int a = 0; a < 4; a++)
     w[a] = g.cov(a, 0) * v[0] + g.cov(a, 1) * v[1] + g.cov(a, 2) * v[2] + g.cov(a, 3) * v[3];
+}
+
+template <class T>
+__device__ __forceinline__ void lower4(const T *v, const GeomFlat &, T *w)
+{
+  w[0] = -v[0];
+  w[1] = v[1];
+  w[2] = v[2];
+  w[3] = v[3];
+}
+__device__ __forceinline__ void lower4(const double *v, const GeomAxi &g, double *w)
+{
+  w[0] = g.c00 * v[0] + g.c01 * v[1] + g.c03 * v[3];
+  w[1] = g.c01 * v[0] + g.c11 * v[1] + g.c13 * v[3];
+  w[2] = g.c22 * v[2];
+  w[3] = g.c03 * v[0] + g.c13 * v[1] + g.c33 * v[3];
 }
 
 __device__ __forceinline__ void raise4(const double *v, const Geom &g, double *w)  // metric.c:362
@@ -122,6 +175,16 @@ __device__ __forceinline__ T quad3(const GT &g, T a, T b, T c)
          2 * (g.cov(1, 2) * a * b + g.cov(1, 3) * a * c + g.cov(2, 3) * b * c);
 }
 
+template <class T>
+__device__ __forceinline__ T quad3(const GeomFlat &, T a, T b, T c)
+{
+  return a * a + b * b + c * c;
+}
+__device__ __forceinline__ double quad3(const GeomAxi &g, double a, double b, double c)
+{
+  return g.c11 * a * a + g.c22 * b * b + g.c33 * c * c + 2 * (g.c13 * a * c);
+}
+
 template <class T, class GT>
 __device__ __forceinline__ int gamma_calc(const T *pr, const GT &g, T *gamma)  // phys.c:244-270
 {
@@ -137,6 +200,31 @@ __device__ __forceinline__ int gamma_calc(const T *pr, const GT &g, T *gamma)  /
   return 0;
 }
 
+// ucon_calc (phys.c:216) from gamma
+template <class T, class GT>
+__device__ __forceinline__ void ucon_of(const T *pr, T gamma, const GT &g, T *ucon)
+{
+  ucon[0] = gamma * g.nc(0);
+  ucon[1] = pr[U1] - ucon[0] * g.bet(0);
+  ucon[2] = pr[U2] - ucon[0] * g.bet(1);
+  ucon[3] = pr[U3] - ucon[0] * g.bet(2);
+}
+template <class T>
+__device__ __forceinline__ void ucon_of(const T *pr, T gamma, const GeomFlat &, T *ucon)
+{
+  ucon[0] = gamma;
+  ucon[1] = pr[U1];
+  ucon[2] = pr[U2];
+  ucon[3] = pr[U3];
+}
+__device__ __forceinline__ void ucon_of(const double *pr, double gamma, const GeomAxi &g, double *ucon)
+{
+  ucon[0] = gamma * g.nc0;
+  ucon[1] = pr[U1] - ucon[0] * g.b0;
+  ucon[2] = pr[U2];
+  ucon[3] = pr[U3];
+}
+
 // get_state (phys.c:199), with ucon_calc (phys.c:216) and bcon_calc (phys.c:75).
 // Returns 1 if gamma_calc failed (the caller books FAIL_GAMMA_CALC).
 template <class T, class GT>
@@ -144,10 +232,7 @@ __device__ __forceinline__ int get_state(const T *pr, const GT &g, T gam, StateT
 {
   T gamma;
   const int bad = gamma_calc(pr, g, &gamma);
-  q.ucon[0] = gamma * g.nc(0);
-  q.ucon[1] = pr[U1] - q.ucon[0] * g.bet(0);
-  q.ucon[2] = pr[U2] - q.ucon[0] * g.bet(1);
-  q.ucon[3] = pr[U3] - q.ucon[0] * g.bet(2);
+  ucon_of(pr, gamma, g, q.ucon);
   lower4(q.ucon, g, q.ucov);
   const T inv_ut = T(1) / q.ucon[0];
   q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
@@ -190,6 +275,19 @@ __device__ __forceinline__ void primtoflux(const double *pr, const State &q, int
   for (int l = 0; l < HG_NPR; l++) f[l] *= g.g;
 }
 
+// gcon[0][js] + x of vchar_fast: known to be x for js = x2, x3 and in flat space
+template <class T, class GT>
+__device__ __forceinline__ T add_con0(const GT &g, int js, T x)
+{
+  return g.con(0, js) + x;
+}
+template <class T>
+__device__ __forceinline__ T add_con0(const GeomFlat &, int, T x)
+{
+  return x;
+}
+__device__ __forceinline__ double add_con0(const GeomAxi &g, int js, double x) { return js == 1 ? g.n0d + x : x; }
+
 template <class T, class GT>
 __device__ __forceinline__ void vchar_fast(const StateT<T> &q, const GT &g, int js, T gam, T *vmax,
                                            T *vmin)  // phys.c:432-501
@@ -201,7 +299,7 @@ __device__ __forceinline__ void vchar_fast(const StateT<T> &q, const GT &g, int 
   const T Bu2 = q.ucon[0] * q.ucon[0];
   const T AuBu = q.ucon[js] * q.ucon[0];
   const T A = Bu2 - (g.con(0, 0) + Bu2) * cms2;
-  const T B = AuBu - (g.con(0, js) + AuBu) * cms2;
+  const T B = AuBu - add_con0(g, js, AuBu) * cms2;
   const T C = Au2 - (g.con(js, js) + Au2) * cms2;
   T discr = B * B - A * C;
   if (discr < T(0)) discr = T(0);
