@@ -379,7 +379,11 @@ static bool flat_geom(const double *s)
       const double n = s[a * 4 + b], c = s[16 + a * 4 + b];
       if (a == b ? (n != e || c != e) : !(plus_zero(n) && plus_zero(c))) return false;
     }
-  return s[32] == 1. && s[38] == 1. && s[35] == 0. && s[36] == 0. && s[37] == 0.;
+  for (int f : {32, 33, 34, 38})  // sqrt(-g), its inverse, alpha, ncon[0]
+    if (s[f] != 1.) return false;
+  for (int f : {35, 36, 37, 39, 40, 41})  // beta, ncon[1..3]
+    if (s[f] != 0.) return false;
+  return true;
 }
 static bool axi_geom(const double *s)
 {

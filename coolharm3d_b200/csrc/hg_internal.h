@@ -41,6 +41,8 @@ struct Geom {
   __host__ __device__ double nc(int a) const { return ncon[a]; }
   __host__ __device__ double bet(int a) const { return beta[a]; }
   __host__ __device__ double det() const { return g; }
+  __host__ __device__ double ginv() const { return g_inv; }
+  __host__ __device__ double lapse() const { return alpha; }
 };
 
 // What a scan of the uploaded geometry found (hg_set_geometry): FLAT is the

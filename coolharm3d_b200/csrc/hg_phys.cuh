@@ -99,12 +99,16 @@ __device__ __forceinline__ void load_geom(const GridDev &G, int pos, int i, int 
 }
 
 // Geometries whose zeros are known at compile time (HG_GK_FLAT, HG_GK_AXI),
-// for the face fluxes: the overloads below leave out the products with a
-// zero entry.  For finite states a sum without its +-0 terms is the same
-// number (only the sign of a zero result can differ), so face_flux checks
-// that the states are finite and the sums that consume its fluxes
-// (update_zone, k_emf) start from or add +0, which takes the sign back.
+// for the face fluxes, the conserved update and the inversion: the overloads
+// below leave out the products with a zero entry.  For finite states a sum
+// without its +-0 terms is the same number (only the sign of a zero result
+// can differ), so face_flux and cons_zone check that the states are finite
+// and the sums that consume their results (update_zone, k_emf) start from or
+// add +0, which takes the sign back; k_update_c2p checks its conserved
+// variables.
 struct GeomFlat {
+  __device__ double ginv() const { return 1.; }
+  __device__ double lapse() const { return 1.; }
   __device__ double con(int a, int b) const { return a == b ? (a == 0 ? -1. : 1.) : 0.; }
   __device__ double det() const { return 1.; }
 };
@@ -133,6 +137,51 @@ __device__ __forceinline__ void load_face_geom(const GridDev &G, int i, int j, G
   g.g = __ldg(t + 32 * s);
   g.b0 = __ldg(t + 35 * s);
   g.nc0 = __ldg(t + 38 * s);
+}
+
+// the centre's entries: of gcov and the normal, for the state ...
+__device__ __forceinline__ void load_cent_geom(const GridDev &G, int i, int j, GeomAxi &g)
+{
+  const double *t = G.geomT + ((long)3 * G.T[1] + j) * G.T[0] + i;
+  const long s = G.gS;
+  g.c00 = __ldg(t + 16 * s);
+  g.c01 = __ldg(t + 17 * s);
+  g.c03 = __ldg(t + 19 * s);
+  g.c11 = __ldg(t + 21 * s);
+  g.c13 = __ldg(t + 23 * s);
+  g.c22 = __ldg(t + 26 * s);
+  g.c33 = __ldg(t + 31 * s);
+  g.n00 = g.n0d = g.ndd = 0.;  // not read
+  g.g = __ldg(t + 32 * s);
+  g.b0 = __ldg(t + 35 * s);
+  g.nc0 = __ldg(t + 38 * s);
+}
+// ... and those the inversion reads
+struct GeomAxiInv {
+  double c11, c13, c22, c33;            // gcov
+  double n00, n01, n11, n13, n22, n33;  // gcon
+  double g_inv, alpha, ncon[4];
+  __device__ double ginv() const { return g_inv; }
+  __device__ double lapse() const { return alpha; }
+};
+__device__ __forceinline__ void load_inv_geom(const GridDev &G, int i, int j, GeomAxiInv &g)
+{
+  const double *t = G.geomT + ((long)3 * G.T[1] + j) * G.T[0] + i;
+  const long s = G.gS;
+  g.c11 = __ldg(t + 21 * s);
+  g.c13 = __ldg(t + 23 * s);
+  g.c22 = __ldg(t + 26 * s);
+  g.c33 = __ldg(t + 31 * s);
+  g.n00 = __ldg(t);
+  g.n01 = __ldg(t + s);
+  g.n11 = __ldg(t + 5 * s);
+  g.n13 = __ldg(t + 7 * s);
+  g.n22 = __ldg(t + 10 * s);
+  g.n33 = __ldg(t + 15 * s);
+  g.g_inv = __ldg(t + 33 * s);
+  g.alpha = __ldg(t + 34 * s);
+#pragma unroll
+  for (int a = 1; a < 4; a++) g.ncon[a] = __ldg(t + (38 + a) * s);
 }
 
 template <class T, class GT>
@@ -166,6 +215,25 @@ __device__ __forceinline__ void raise4(const double *v, const Geom &g, double *w
     w[a] = g.gcon[a][0] * v[0] + g.gcon[a][1] * v[1] + g.gcon[a][2] * v[2] + g.gcon[a][3] * v[3];
 }
 
+__device__ __forceinline__ void raise4(const double *v, const GeomFlat &, double *w)
+{
+  w[0] = -v[0];
+  w[1] = v[1];
+  w[2] = v[2];
+  w[3] = v[3];
+}
+__device__ __forceinline__ void raise4(const double *v, const GeomAxiInv &g, double *w)
+{
+  w[0] = g.n00 * v[0] + g.n01 * v[1];
+  w[1] = g.n01 * v[0] + g.n11 * v[1] + g.n13 * v[3];
+  w[2] = g.n22 * v[2];
+  w[3] = g.n13 * v[1] + g.n33 * v[3];
+}
+// x + ncon[a] y of the inversion's last lines
+__device__ __forceinline__ double add_ncon(const Geom &g, int a, double x, double y) { return x + g.ncon[a] * y; }
+__device__ __forceinline__ double add_ncon(const GeomAxiInv &g, int a, double x, double y) { return x + g.ncon[a] * y; }
+__device__ __forceinline__ double add_ncon(const GeomFlat &, int, double x, double) { return x; }
+
 // The gcov-weighted spatial quadratic form of gamma_calc (phys.c:249-255),
 // Utoprim_new_body's Bsq and utsq (utoprim_2d_fast.c:255-304).
 template <class T, class GT>
@@ -180,9 +248,15 @@ __device__ __forceinline__ T quad3(const GeomFlat &, T a, T b, T c)
 {
   return a * a + b * b + c * c;
 }
-__device__ __forceinline__ double quad3(const GeomAxi &g, double a, double b, double c)
+template <class GA>
+__device__ __forceinline__ double quad3_axi(const GA &g, double a, double b, double c)
 {
   return g.c11 * a * a + g.c22 * b * b + g.c33 * c * c + 2 * (g.c13 * a * c);
+}
+__device__ __forceinline__ double quad3(const GeomAxi &g, double a, double b, double c) { return quad3_axi(g, a, b, c); }
+__device__ __forceinline__ double quad3(const GeomAxiInv &g, double a, double b, double c)
+{
+  return quad3_axi(g, a, b, c);
 }
 
 template <class T, class GT>
@@ -258,7 +332,8 @@ __device__ __forceinline__ void mhd_row(const State &q, int dir, double *mhd)  /
   mhd[dir] += q.ptot;
 }
 
-__device__ __forceinline__ void primtoflux(const double *pr, const State &q, int dir, const Geom &g,
+template <class GT>
+__device__ __forceinline__ void primtoflux(const double *pr, const State &q, int dir, const GT &g,
                                            double *f)  // phys.c:28-63
 {
   double mhd[4];
@@ -272,7 +347,7 @@ __device__ __forceinline__ void primtoflux(const double *pr, const State &q, int
   f[B2] = q.bcon[2] * q.ucon[dir] - q.bcon[dir] * q.ucon[2];
   f[B3] = q.bcon[3] * q.ucon[dir] - q.bcon[dir] * q.ucon[3];
 #pragma unroll
-  for (int l = 0; l < HG_NPR; l++) f[l] *= g.g;
+  for (int l = 0; l < HG_NPR; l++) f[l] *= g.det();
 }
 
 // gcon[0][js] + x of vchar_fast: known to be x for js = x2, x3 and in flat space
@@ -457,11 +532,12 @@ __device__ __forceinline__ void ppm_zone(int rt, const T *y, T *ln, T *rn)
 
 // ---------------------------------------------------------------------------
 // Con2prim (utoprim_2d_fast.c:135-740).  Returns the reference's codes.
-__device__ __forceinline__ int utoprim_2d(const double *U, const Geom &g, double gam, double *prim, double *gamma_out,
+template <class GT>
+__device__ __forceinline__ int utoprim_2d(const double *U, const GT &g, double gam, double *prim, double *gamma_out,
                                           double *bsq_out)
 {
   if (U[0] <= 0.) return -100;
-  const double inv_gdet = g.g_inv, alpha = g.alpha, gf = alpha * inv_gdet;
+  const double inv_gdet = g.ginv(), alpha = g.lapse(), gf = alpha * inv_gdet;
   prim[B1] = U[B1] * inv_gdet;
   prim[B2] = U[B2] * inv_gdet;
   prim[B3] = U[B3] * inv_gdet;
@@ -564,9 +640,9 @@ __device__ __forceinline__ int utoprim_2d(const double *U, const Geom &g, double
   *bsq_out = Bsq * (1. - vsq) + QdB_o_W * QdB_o_W;
   prim[RHO] = rho0;
   prim[UU] = u;
-  prim[U1] = g_o_WBsq * (Qcon[1] + g.ncon[1] * Qdotn + QdB_o_W * Bcon[1]);
-  prim[U2] = g_o_WBsq * (Qcon[2] + g.ncon[2] * Qdotn + QdB_o_W * Bcon[2]);
-  prim[U3] = g_o_WBsq * (Qcon[3] + g.ncon[3] * Qdotn + QdB_o_W * Bcon[3]);
+  prim[U1] = g_o_WBsq * (add_ncon(g, 1, Qcon[1], Qdotn) + QdB_o_W * Bcon[1]);
+  prim[U2] = g_o_WBsq * (add_ncon(g, 2, Qcon[2], Qdotn) + QdB_o_W * Bcon[2]);
+  prim[U3] = g_o_WBsq * (add_ncon(g, 3, Qcon[3], Qdotn) + QdB_o_W * Bcon[3]);
   return 0;
 }
 
