@@ -215,6 +215,9 @@ __device__ __forceinline__ void face_prims(const GridDev &G, const double *__res
 // finite (known-zero geometries), or to 1.
 __device__ __forceinline__ bool is_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
+__device__ __forceinline__ bool all_ok(const SlowDiv &) { return true; }
+__device__ __forceinline__ bool all_ok(const FastDiv &dv) { return dv.ok; }
+
 template <int d, class GT>
 __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, const double *pr, const GT &g,
                                             int i, int j, int k, unsigned int mult, double *__restrict__ Fd, long o,
@@ -223,7 +226,12 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
   constexpr int dim = d + 1;
   constexpr bool full = std::is_same<GT, Geom>::value;
   State ql, qr;
-  const int badl = get_state(pl, g, G.gam, ql), badr = get_state(pr, g, G.gam, qr);
+  double cmaxl, cminl, cmaxr, cminr;
+  typename std::conditional<full, SlowDiv, FastDiv>::type dv;
+  double gml, gmr;
+  const int badl = gamma_calc(pl, g, &gml), badr = gamma_calc(pr, g, &gmr);
+  state_of(pl, gml, g, G.gam, ql, dv);
+  state_of(pr, gmr, g, G.gam, qr, dv);
   if (full) {
     if (badl) book_face(G, i, j, k, mult);
     if (badr) book_face(G, i, j, k, mult);
@@ -232,9 +240,13 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
     // ucon[0] and bsq are infinite or NaN if any of ucon, bcon is
     *fin = !(badl | badr) && is_finite((ql.ucon[0] + ql.bsq) + (qr.ucon[0] + qr.bsq));
   }
-  double cmaxl, cminl, cmaxr, cminr;
-  vchar_fast(ql, g, dim, G.gam, &cmaxl, &cminl);
-  vchar_fast(qr, g, dim, G.gam, &cmaxr, &cminr);
+  {
+    double Al, Bl, Ar, Br;
+    const double dl = vchar_discr(ql, g, dim, G.gam, &Al, &Bl, dv), dr = vchar_discr(qr, g, dim, G.gam, &Ar, &Br, dv);
+    const double rl = sqrt(dl), rr = sqrt(dr);
+    vchar_speeds(Al, Bl, rl, &cmaxl, &cminl, dv);
+    vchar_speeds(Ar, Br, rr, &cmaxr, &cminr, dv);
+  }
   const double a0 = 0. > cmaxl ? 0. : cmaxl;
   const double cmax = fabs(a0 > cmaxr ? a0 : cmaxr);
   const double a1 = 0. > -cminl ? 0. : -cminl;
@@ -243,12 +255,26 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
   const double gg = g.det();
   if (G.flux == 1) {
     const double den = cmax + cmin + HG_SMALL;
+    double num[HG_NPR];
 #pragma unroll
     for (int l = 0; l < HG_NPR; l++) {
-      if (l == B1 + d && !(full && all)) continue;
       const double Ul = flux_comp(pl, ql, 0, gg, l), Ur = flux_comp(pr, qr, 0, gg, l);
       const double Fl = flux_comp(pl, ql, dim, gg, l), Fr = flux_comp(pr, qr, dim, gg, l);
-      Fd[l * G.S + o] = (cmax * Fl + cmin * Fr - cmax * cmin * (Ur - Ul)) / den;
+      num[l] = cmax * Fl + cmin * Fr - cmax * cmin * (Ur - Ul);
+      if (full && (l != B1 + d || all)) Fd[l * G.S + o] = num[l] / den;
+    }
+    if (!full) {
+      FastDiv fd;
+      const double y = fd.rcp(den);
+#pragma unroll
+      for (int l = 0; l < HG_NPR; l++)
+        if (l != B1 + d) Fd[l * G.S + o] = fd.by(num[l], den, y);
+      // fields decay to the smallest numbers ahead of where they flow: only
+      // the quotients are formed again (the whole face again: 4.69 ms)
+      if (!fd.ok)
+#pragma unroll
+        for (int l = 0; l < HG_NPR; l++)
+          if (l != B1 + d) Fd[l * G.S + o] = num[l] / den;
     }
   } else {
 #pragma unroll
@@ -259,6 +285,7 @@ __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, 
       Fd[l * G.S + o] = 0.5 * (Fl + Fr - ctop * (Ur - Ul));
     }
   }
+  if (!full) *fin &= all_ok(dv);
   return ctop;
 }
 

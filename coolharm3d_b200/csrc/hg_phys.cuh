@@ -98,6 +98,52 @@ __device__ __forceinline__ void load_geom(const GridDev &G, int pos, int i, int 
   g.ncon[3] = __ldg(t + 41 * s);
 }
 
+// Divisions correctly rounded without a branch each, so that the compiler can
+// interleave them: x / y is a serial chain of its own between two branches.
+// P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor (IBM J. Res. Dev. 34, 1990): from a reciprocal y
+// within one unit in the last place of 1/b, y += y (1 - b y) with fused
+// multiply-adds is the correctly rounded reciprocal unless b's mantissa is
+// all ones; with it, a quotient q within one unit becomes the correctly
+// rounded one by q += y (a - b q), whose remainder is exact.  The seed is
+// rcp.approx (20 bits): two Newton steps reach one unit in the last place,
+// a third rounds it.  ok is cleared where the theorems do not apply: b
+// outside [2^-400, 2^400] or of 53 ones (its low word is looked at), a
+// neither 0 nor within [2^-500, 2^500] (no product or remainder underflows).
+// The caller then takes the plain divisions (SlowDiv) instead.  In the flux
+// kernels the five divisions of the two states and the seven of the HLL sum
+// so share one chain: flux of a 128^3 flat step 1.27 -> 1.18 ms, of a
+// 192x192x128 torus step 3.23 -> 3.14, of 1024 zones in a line 10 -> 8.5 us.
+struct SlowDiv {
+  template <class T>
+  __device__ T rcp(T b) { return T(1) / b; }
+  template <class T>
+  __device__ T div(T a, T b) { return a / b; }
+};
+struct FastDiv {
+  bool ok = true;
+  __device__ double rcp(double b)
+  {
+    const unsigned h = __double2hiint(b) & 0x7fffffffu;
+    ok &= h - ((1023u - 400u) << 20) < (800u << 20) && __double2loint(b) != -1;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __fma_rn(__fma_rn(-b, y, 1.), y, y);
+    y = __fma_rn(__fma_rn(-b, y, 1.), y, y);
+    return __fma_rn(__fma_rn(-b, y, 1.), y, y);
+  }
+  // a / b with y = rcp(b); 0 for a zero (its sign is not kept)
+  __device__ double by(double a, double b, double y)
+  {
+    const unsigned h = __double2hiint(a) & 0x7fffffffu;
+    ok &= h - ((1023u - 500u) << 20) < (1000u << 20) || (h | (unsigned)__double2loint(a)) == 0u;
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+  }
+  __device__ double div(double a, double b) { return by(a, b, rcp(b)); }
+};
+
 // Geometries whose zeros are known at compile time (HG_GK_FLAT, HG_GK_AXI),
 // for the face fluxes, the conserved update and the inversion: the overloads
 // below leave out the products with a zero entry.  For finite states a sum
@@ -301,14 +347,12 @@ __device__ __forceinline__ void ucon_of(const double *pr, double gamma, const Ge
 
 // get_state (phys.c:199), with ucon_calc (phys.c:216) and bcon_calc (phys.c:75).
 // Returns 1 if gamma_calc failed (the caller books FAIL_GAMMA_CALC).
-template <class T, class GT>
-__device__ __forceinline__ int get_state(const T *pr, const GT &g, T gam, StateT<T> &q)
+template <class T, class GT, class DV>
+__device__ __forceinline__ void state_of(const T *pr, T gamma, const GT &g, T gam, StateT<T> &q, DV &dv)
 {
-  T gamma;
-  const int bad = gamma_calc(pr, g, &gamma);
   ucon_of(pr, gamma, g, q.ucon);
   lower4(q.ucon, g, q.ucov);
-  const T inv_ut = T(1) / q.ucon[0];
+  const T inv_ut = dv.rcp(q.ucon[0]);
   q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
   q.bcon[1] = (pr[B1] + q.bcon[0] * q.ucon[1]) * inv_ut;
   q.bcon[2] = (pr[B2] + q.bcon[0] * q.ucon[2]) * inv_ut;
@@ -318,6 +362,14 @@ __device__ __forceinline__ int get_state(const T *pr, const GT &g, T gam, StateT
   q.p = (gam - T(1)) * pr[UU];
   q.eta = q.p + pr[RHO] + pr[UU] + q.bsq;
   q.ptot = q.p + T(0.5) * q.bsq;
+}
+template <class T, class GT>
+__device__ __forceinline__ int get_state(const T *pr, const GT &g, T gam, StateT<T> &q)
+{
+  T gamma;
+  const int bad = gamma_calc(pr, g, &gamma);
+  SlowDiv dv;
+  state_of(pr, gamma, g, gam, q, dv);
   return bad;
 }
 
@@ -363,11 +415,12 @@ __device__ __forceinline__ T add_con0(const GeomFlat &, int, T x)
 }
 __device__ __forceinline__ double add_con0(const GeomAxi &g, int js, double x) { return js == 1 ? g.n0d + x : x; }
 
-template <class T, class GT>
-__device__ __forceinline__ void vchar_fast(const StateT<T> &q, const GT &g, int js, T gam, T *vmax,
-                                           T *vmin)  // phys.c:432-501
+// vchar_fast, phys.c:432-501, in two parts: the square of the discriminant's
+// root, then the speeds from the root
+template <class T, class GT, class DV>
+__device__ __forceinline__ T vchar_discr(const StateT<T> &q, const GT &g, int js, T gam, T *A_out, T *B_out, DV &dv)
 {
-  T cms2 = (gam * q.p + q.bsq) / q.eta;
+  T cms2 = dv.div(gam * q.p + q.bsq, q.eta);
   if (cms2 < T(0)) cms2 = T(HG_SMALL);
   else if (cms2 > T(1)) cms2 = T(1);
   const T Au2 = q.ucon[js] * q.ucon[js];
@@ -378,10 +431,16 @@ __device__ __forceinline__ void vchar_fast(const StateT<T> &q, const GT &g, int 
   const T C = Au2 - (g.con(js, js) + Au2) * cms2;
   T discr = B * B - A * C;
   if (discr < T(0)) discr = T(0);
-  discr = sqrt(discr);
-  const T denom = T(1) / A;
-  const T vp = -(-B + discr) * denom;
-  const T vm = -(-B - discr) * denom;
+  *A_out = A;
+  *B_out = B;
+  return discr;
+}
+template <class T, class DV>
+__device__ __forceinline__ void vchar_speeds(T A, T B, T root, T *vmax, T *vmin, DV &dv)
+{
+  const T denom = dv.rcp(A);
+  const T vp = -(-B + root) * denom;
+  const T vm = -(-B - root) * denom;
   if (vp > vm) {
     *vmax = vp;
     *vmin = vm;
@@ -389,6 +448,14 @@ __device__ __forceinline__ void vchar_fast(const StateT<T> &q, const GT &g, int 
     *vmax = vm;
     *vmin = vp;
   }
+}
+template <class T, class GT>
+__device__ __forceinline__ void vchar_fast(const StateT<T> &q, const GT &g, int js, T gam, T *vmax, T *vmin)
+{
+  SlowDiv dv;
+  T A, B;
+  const T discr = vchar_discr(q, g, js, gam, &A, &B, dv);
+  vchar_speeds(A, B, T(sqrt(discr)), vmax, vmin, dv);
 }
 
 // One component of primtoflux(pr, q, dir) (phys.c:28-63), same operations.
