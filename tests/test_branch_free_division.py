@@ -17,10 +17,10 @@ pytestmark = pytest.mark.gpu
 
 def wide_state(f, lo, seed):
     """The fixture's state with fields scaled by 1 .. 10^lo, zone by zone, some
-    zero, and densities by 1 .. 1e-6."""
+    zero, and densities by 1 .. 1e-6; the copies of a single zone alike."""
     rng = np.random.default_rng(seed)
     p = np.array(f["p0"])
-    s = p.shape[:3]
+    s = tuple(m if n > 1 else 1 for m, n in zip(p.shape, f["n"]))
     p[..., 5:] *= (10.0 ** rng.uniform(lo, 0, s) * (rng.random(s) > 0.2))[..., None]
     p[..., :2] *= (10.0 ** rng.uniform(-6, 0, s))[..., None]
     p[..., 2:5] *= (10.0 ** rng.uniform(lo, 0, s))[..., None]
