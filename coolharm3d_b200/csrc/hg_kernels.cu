@@ -815,6 +815,7 @@ __global__ void __launch_bounds__(HG_BLK, HG_C2P_BLOCKS(GM)) k_update_c2p(const 
     }
     double gamma = 0., bsq = 0.;
     int ret;
+    FastDiv dv;  // where it does not apply, k_fallback repeats the inversion with plain divisions
     if (GM >= HG_GM_FLAT) {
       // variables that are not finite meet every entry in k_fallback, which
       // repeats the inversion: 0 * inf matters there
@@ -824,20 +825,21 @@ __global__ void __launch_bounds__(HG_BLK, HG_C2P_BLOCKS(GM)) k_update_c2p(const 
       ret = 1;
       if (is_finite(sum)) {
         if (GM == HG_GM_FLAT) {
-          ret = utoprim_2d(U, GeomFlat(), G.gam, pf, &gamma, &bsq);
+          ret = utoprim_2d(U, GeomFlat(), G.gam, pf, &gamma, &bsq, dv);
         } else {
           GeomAxiInv g;
           load_inv_geom(G, i, j, g);
-          ret = utoprim_2d(U, g, G.gam, pf, &gamma, &bsq);
+          ret = utoprim_2d(U, g, G.gam, pf, &gamma, &bsq, dv);
         }
       }
     } else if (GM == HG_GM_CONST) {
-      ret = utoprim_2d(U, G.g0, G.gam, pf, &gamma, &bsq);
+      ret = utoprim_2d(U, G.g0, G.gam, pf, &gamma, &bsq, dv);
     } else {
       Geom g;
       load_geom(G, 3, i, j, g, k, sub + 1);
-      ret = utoprim_2d(U, g, G.gam, pf, &gamma, &bsq);
+      ret = utoprim_2d(U, g, G.gam, pf, &gamma, &bsq, dv);
     }
+    if (!dv.ok) ret = 1;
     const bool ee = G.use_ee && ((pf[UU] < HG_BETA_MIN * bsq) || (pf[RHO] < HG_BETA_MIN * bsq));
     if (ret != 0 || check_gamma(gamma) == 2 || ee) {
       // rest of the recover_primitives() tree: queue the zone
@@ -993,7 +995,8 @@ __global__ void __launch_bounds__(HG_BLK) k_fallback(GridDev G, int sub, double 
     if (G.mdim == 3) load_geom(G, 3, i, j, g_old, k, 0);  // geom_old of recover_primitives: n_beg
     else g_old = g;
     double gamma = 0., bsq = 0.;
-    int ret = utoprim_2d(U, g, G.gam, pf, &gamma, &bsq);
+    SlowDiv dv;
+    int ret = utoprim_2d(U, g, G.gam, pf, &gamma, &bsq, dv);
     if ((!ret) && (check_gamma(gamma) == 2)) {
       for (int l = 0; l < B1; l++) pf[l] = pg[l];
       ret = 1;
