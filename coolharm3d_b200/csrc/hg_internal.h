@@ -54,6 +54,17 @@ struct Geom {
 #define HG_GK_FLAT 1
 #define HG_GK_AXI 2
 
+// The face geometries the flux kernels are built for: HG_GM_CONST one struct
+// in the constant bank (metric_dim 0), HG_GM_TAB the (i, j) tables
+// (metric_dim 2), HG_GM_DYN a time level (metric_dim 3), all with every
+// entry; HG_GM_FLAT and HG_GM_AXI with the zeros of HG_GK_FLAT / HG_GK_AXI
+// left out.
+#define HG_GM_CONST 0
+#define HG_GM_TAB 2
+#define HG_GM_DYN 3
+#define HG_GM_FLAT 4
+#define HG_GM_AXI 5
+
 // metric_dim 3 (the time-dependent metric path): the spacetime and the
 // COORD_DIAGONAL3 coordinate parameters its geometry is evaluated from.
 struct DynMetric {

@@ -46,7 +46,7 @@
 namespace hg {
 // the FP32 flux kernels of the mixed form (hg_mixed.cu)
 void launch_flux_f32(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int d, const int *lo, const int *n,
-                     unsigned int mult, int slot);
+                     unsigned int mult, int slot, int all);
 void launch_to_f32(const GridDev &G, int grid, cudaStream_t s, const double *src);
 }  // namespace hg
 
@@ -197,17 +197,6 @@ __device__ __forceinline__ void face_prims(const GridDev &G, const double *__res
 }
 
 // ---------------------------------------------------------------------------
-// The face geometries the flux kernels are built for: HG_GM_CONST one struct
-// in the constant bank (metric_dim 0), HG_GM_TAB the (i, j) tables
-// (metric_dim 2), HG_GM_DYN a time level (metric_dim 3), all with every
-// entry; HG_GM_FLAT and HG_GM_AXI with the zeros of HG_GK_FLAT / HG_GK_AXI
-// left out.
-#define HG_GM_CONST 0
-#define HG_GM_TAB 2
-#define HG_GM_DYN 3
-#define HG_GM_FLAT 4
-#define HG_GM_AXI 5
-
 // HLL/LF flux of a face from its two states; writes the 8 components and
 // returns ctop.  Component by component, so no 32-value temporaries.  The
 // normal field component is left out unless `all` is set: flux-CT replaces
@@ -1701,7 +1690,7 @@ static void launch_flux_dir(const GridDev &G, const LaunchCfg &L, cudaStream_t s
     }
     mark(R, KC_FLUX, s);
     if (G.prec == HG_PREC_MIXED) {
-      launch_flux_f32(G, L, s, d, lo, n, mult, slot);  // reads G.p32, filled from ph
+      launch_flux_f32(G, L, s, d, lo, n, mult, slot, all);  // reads G.p32, filled from ph
       return;
     }
 #define HG_FLUX(RSV, MD, DD) \

@@ -184,19 +184,23 @@ struct FastDiv {
 // and the sums that consume their results (update_zone, k_emf) start from or
 // add +0, which takes the sign back; k_update_c2p checks its conserved
 // variables.
-struct GeomFlat {
-  __device__ double ginv() const { return 1.; }
-  __device__ double lapse() const { return 1.; }
-  __device__ double con(int a, int b) const { return a == b ? (a == 0 ? -1. : 1.) : 0.; }
-  __device__ double det() const { return 1.; }
+template <class T>
+struct GeomFlatT {
+  __device__ T ginv() const { return T(1); }
+  __device__ T lapse() const { return T(1); }
+  __device__ T con(int a, int b) const { return a == b ? (a == 0 ? T(-1) : T(1)) : T(0); }
+  __device__ T det() const { return T(1); }
 };
-struct GeomAxi {
-  double c00, c01, c03, c11, c13, c22, c33;  // gcov
-  double n00, n0d, ndd;                      // gcon of the face's direction d
-  double nc0, b0, g;                         // ncon[0], beta[0], sqrt(-g)
-  __device__ double con(int a, int b) const { return a == 0 ? (b == 0 ? n00 : n0d) : ndd; }
-  __device__ double det() const { return g; }
+typedef GeomFlatT<double> GeomFlat;
+template <class T>
+struct GeomAxiT {
+  T c00, c01, c03, c11, c13, c22, c33;  // gcov
+  T n00, n0d, ndd;                      // gcon of the face's direction d
+  T nc0, b0, g;                         // ncon[0], beta[0], sqrt(-g)
+  __device__ T con(int a, int b) const { return a == 0 ? (b == 0 ? n00 : n0d) : ndd; }
+  __device__ T det() const { return g; }
 };
+typedef GeomAxiT<double> GeomAxi;
 template <int d>
 __device__ __forceinline__ void load_face_geom(const GridDev &G, int i, int j, GeomAxi &g)
 {
@@ -271,14 +275,15 @@ __device__ __forceinline__ void lower4(const T *v, const GT &g, T *w)  // metric
 }
 
 template <class T>
-__device__ __forceinline__ void lower4(const T *v, const GeomFlat &, T *w)
+__device__ __forceinline__ void lower4(const T *v, const GeomFlatT<T> &, T *w)
 {
   w[0] = -v[0];
   w[1] = v[1];
   w[2] = v[2];
   w[3] = v[3];
 }
-__device__ __forceinline__ void lower4(const double *v, const GeomAxi &g, double *w)
+template <class T>
+__device__ __forceinline__ void lower4(const T *v, const GeomAxiT<T> &g, T *w)
 {
   w[0] = g.c00 * v[0] + g.c01 * v[1] + g.c03 * v[3];
   w[1] = g.c01 * v[0] + g.c11 * v[1] + g.c13 * v[3];
@@ -322,16 +327,20 @@ __device__ __forceinline__ T quad3(const GT &g, T a, T b, T c)
 }
 
 template <class T>
-__device__ __forceinline__ T quad3(const GeomFlat &, T a, T b, T c)
+__device__ __forceinline__ T quad3(const GeomFlatT<T> &, T a, T b, T c)
 {
   return a * a + b * b + c * c;
 }
-template <class GA>
-__device__ __forceinline__ double quad3_axi(const GA &g, double a, double b, double c)
+template <class T, class GA>
+__device__ __forceinline__ T quad3_axi(const GA &g, T a, T b, T c)
 {
   return g.c11 * a * a + g.c22 * b * b + g.c33 * c * c + 2 * (g.c13 * a * c);
 }
-__device__ __forceinline__ double quad3(const GeomAxi &g, double a, double b, double c) { return quad3_axi(g, a, b, c); }
+template <class T>
+__device__ __forceinline__ T quad3(const GeomAxiT<T> &g, T a, T b, T c)
+{
+  return quad3_axi(g, a, b, c);
+}
 __device__ __forceinline__ double quad3(const GeomAxiInv &g, double a, double b, double c)
 {
   return quad3_axi(g, a, b, c);
@@ -362,14 +371,15 @@ __device__ __forceinline__ void ucon_of(const T *pr, T gamma, const GT &g, T *uc
   ucon[3] = pr[U3] - ucon[0] * g.bet(2);
 }
 template <class T>
-__device__ __forceinline__ void ucon_of(const T *pr, T gamma, const GeomFlat &, T *ucon)
+__device__ __forceinline__ void ucon_of(const T *pr, T gamma, const GeomFlatT<T> &, T *ucon)
 {
   ucon[0] = gamma;
   ucon[1] = pr[U1];
   ucon[2] = pr[U2];
   ucon[3] = pr[U3];
 }
-__device__ __forceinline__ void ucon_of(const double *pr, double gamma, const GeomAxi &g, double *ucon)
+template <class T>
+__device__ __forceinline__ void ucon_of(const T *pr, T gamma, const GeomAxiT<T> &g, T *ucon)
 {
   ucon[0] = gamma * g.nc0;
   ucon[1] = pr[U1] - ucon[0] * g.b0;
@@ -441,11 +451,15 @@ __device__ __forceinline__ T add_con0(const GT &g, int js, T x)
   return g.con(0, js) + x;
 }
 template <class T>
-__device__ __forceinline__ T add_con0(const GeomFlat &, int, T x)
+__device__ __forceinline__ T add_con0(const GeomFlatT<T> &, int, T x)
 {
   return x;
 }
-__device__ __forceinline__ double add_con0(const GeomAxi &g, int js, double x) { return js == 1 ? g.n0d + x : x; }
+template <class T>
+__device__ __forceinline__ T add_con0(const GeomAxiT<T> &g, int js, T x)
+{
+  return js == 1 ? g.n0d + x : x;
+}
 
 // vchar_fast, phys.c:432-501, in two parts: the square of the discriminant's
 // root, then the speeds from the root
