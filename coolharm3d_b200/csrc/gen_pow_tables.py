@@ -12,6 +12,11 @@ value to about 2^-106 relative:
   LN2_256      = log(2)/256 as C1 + C2 + C3, C1 with 32 significant bits so
                  that n*C1 is exact for |n| < 2^21
   INV_LN2_256  = 256/log(2) (only selects the reduction index)
+  FLOG[i]      = 1/c, -log(1/c) as hi (a multiple of 2^-42) + lo, 0; c the
+                 middle of [1 + i/256, 1 + (i+1)/256), but 1 for i = 0 and 2
+                 for i = 255; from i = 106 on (c > sqrt 2) less log(2), the
+                 exponent being one more there   (quick log)
+  FLN2         = log(2) as hi (a multiple of 2^-42) + lo
 
 Usage: python gen_pow_tables.py  (rewrites hg_pow_tables.h beside it)
 """
@@ -48,6 +53,18 @@ def main():
     ln2_hi, ln2_lo = split(ln2)
     inv = float(256 / ln2)
 
+    def coarse(v):
+        hi = float((v * 2**42).to_integral_value()) / 2**42
+        return hi, float(v - Decimal(hi))
+
+    flog = []
+    for i in range(256):
+        c = Decimal(1) if i == 0 else Decimal(2) if i == 255 else 1 + (Decimal(i) + Decimal("0.5")) / 256
+        rc = float(1 / c)
+        hi, lo = coarse(-Decimal(rc).ln() - (ln2 if i >= 106 else 0))
+        flog.append((rc, hi, lo))
+    fln2 = coarse(ln2)
+
     def row(pairs):
         return ",\n".join("  %s, %s" % (a.hex(), b.hex()) for a, b in pairs)
 
@@ -70,12 +87,19 @@ def main():
         out.append("#define HG_POW_%s_LO %s" % (name, lo.hex()))
     for d in (5, 7, 9, 11, 24, 120, 720, 5040, 40320):
         out.append("#define HG_POW_INV%d %s" % (d, float(Decimal(1) / d).hex()))
+    for d in (3, 4, 6, 8):
+        out.append("#define HG_POW_INV%d %s" % (d, float(Decimal(1) / d).hex()))
+    out.append("#define HG_POW_FLN2_HI %s" % fln2[0].hex())
+    out.append("#define HG_POW_FLN2_LO %s" % fln2[1].hex())
     out.append("/* log(1 + k/256), k = %d .. %d */" % (K_LO, K_HI))
     out.append("#define HG_POW_LOGC_TABLE {\\")
     out.append(row(logc).replace("\n", "\\\n") + "}")
     out.append("/* 2^(j/256), j = 0 .. 255 */")
     out.append("#define HG_POW_EXP2_TABLE {\\")
     out.append(row(exp2).replace("\n", "\\\n") + "}")
+    out.append("/* quick log: 1/c, -log(1/c) hi and lo, 0 */")
+    out.append("#define HG_POW_FLOG_TABLE {\\")
+    out.append(",\\\n".join("  %s, %s, %s, 0.0" % (a.hex(), b.hex(), c.hex()) for a, b, c in flog) + "}")
     out.append("#endif")
     with open(os.path.join(HERE, "hg_pow_tables.h"), "w") as f:
         f.write("\n".join(out) + "\n")

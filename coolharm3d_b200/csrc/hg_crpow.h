@@ -26,6 +26,10 @@
  * The leading terms of both series are carried in double-double, the tail
  * in double; the tables log(1 + k/256) and 2^(j/256) are double-double
  * values computed with 80-digit decimal arithmetic (gen_pow_tables.py).
+ * Before that a quick phase of a fifth of the length (hg_pow_quick) computes
+ * x^y to within 2^-68 in single steps of double arithmetic with one low word,
+ * and returns its rounding where no number that close rounds otherwise (all
+ * but one call in 3000).
  * Other inputs (x <= 0, subnormal or infinite x, NaN, |y log x| >= 700) go
  * to the platform's pow(); the step never produces them.
  *
@@ -47,9 +51,11 @@
 
 static const double hg_pow_logc_h[2 * HG_POW_NLOGC] = HG_POW_LOGC_TABLE;
 static const double hg_pow_exp2_h[2 * 256] = HG_POW_EXP2_TABLE;
+static const double hg_pow_flog_h[4 * 256] = HG_POW_FLOG_TABLE;
 #ifdef __CUDACC__
 static __device__ const double hg_pow_logc_d[2 * HG_POW_NLOGC] = HG_POW_LOGC_TABLE;
 static __device__ const double hg_pow_exp2_d[2 * 256] = HG_POW_EXP2_TABLE;
+static __device__ const double hg_pow_flog_d[4 * 256] = HG_POW_FLOG_TABLE;
 #endif
 
 typedef struct {
@@ -80,10 +86,21 @@ HG_PHD hg_dd hg_dd_fast_sum(double a, double b)
   return hg_dd_make(s, b - (s - a));
 }
 
+/* a * b rounded, kept apart from an addition that follows it also where the
+ * compiler fuses multiply-adds */
+HG_PHD double hg_pow_mul(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+
 /* a * b exactly as p + e */
 HG_PHD hg_dd hg_dd_prod(double a, double b)
 {
-  const double p = a * b;
+  const double p = hg_pow_mul(a, b);
   return hg_dd_make(p, fma(a, b, -p));
 }
 
@@ -201,6 +218,67 @@ HG_PHD double hg_dd_exp_rn(hg_dd E)
   return res.hi * hg_pow_from_bits((uint64_t)(q + 1023) << 52);
 }
 
+HG_PHD double hg_pow_flog(int i, int m)
+{
+#ifdef __CUDA_ARCH__
+  return __ldg(hg_pow_flog_d + 4 * i + m);
+#else
+  return hg_pow_flog_h[4 * i + m];
+#endif
+}
+
+/* x^y for a positive normal x and |y| <= 2: 1 and *out the double nearest to
+ * it, or 0 where the quick phase cannot tell (or |y log x| >= 700).
+ *
+ * The two dependent chains of the Newton solves that call it are as long as
+ * the pow, so what counts is its depth: some 60 dependent operations against
+ * 300.  Errors, absolute in E = y log x and relative in the result:
+ *   log: x = 2^e m, m/c = p + pl exactly (c's reciprocal from the table),
+ *     r = p - 1 exact, |r| <= 2^-8.  e log 2 - log(1/c) is exact in its high
+ *     parts (multiples of 2^-42 below 2^10).  The series' r^9/9 < 2^-75 is
+ *     left out, its r^3 term (< 2^-25.5) is rounded to within 2^-76, the
+ *     part pl r^3 of pl's correction < 2^-77: 2^-74 with all roundings.
+ *   exp: |rh| <= log(2)/512 < 2^-9.5, rh^7/5040 < 2^-78 left out; A (< 2^-20)
+ *     and what it is multiplied by and added to rounded to within 2^-70.5.
+ * In all less than 2^-69 (2^-70.3 the largest of 60,000 against 60 digits); the
+ * test allows 2^-65 of a result in [1, 2).  Entropy fix of a 192x192x128 torus
+ * step 0.574 -> 0.520 ms, of a 96x96x64 one 0.295 -> 0.263. */
+HG_PHD int hg_pow_quick(double x, double y, double *out)
+{
+  const uint64_t bits = hg_pow_bits(x);
+  const int i = (int)(bits >> 44) & 255;
+  const double e = (double)((int)(bits >> 52) - 1023 + (i >= 106 ? 1 : 0));
+  const double m = hg_pow_from_bits((bits & 0x000fffffffffffffull) | 0x3ff0000000000000ull);
+  const double rc = hg_pow_flog(i, 0);
+  const double p = hg_pow_mul(m, rc), pl = fma(m, rc, -p), r = p - 1.0, rr = r * r;
+  const hg_dd a = hg_dd_two_sum(e * HG_POW_FLN2_HI + hg_pow_flog(i, 1), r);
+  const hg_dd b = hg_dd_fast_sum(a.hi, -0.5 * rr);
+  const double cub = (r * rr) * ((HG_POW_INV3 - r * HG_POW_INV4) +
+                                 rr * ((HG_POW_INV5 - r * HG_POW_INV6) + rr * (HG_POW_INV7 - r * HG_POW_INV8)));
+  const double low = ((cub - 0.5 * fma(r, r, -rr)) + (pl - pl * (r - rr))) +
+                     ((a.lo + b.lo) + (e * HG_POW_FLN2_LO + hg_pow_flog(i, 2)));
+  const hg_dd L = hg_dd_fast_sum(b.hi, low);
+  const double Eh = hg_pow_mul(y, L.hi);
+  if (!(fabs(Eh) < 700.0)) return 0;
+  const double El = fma(y, L.hi, -Eh) + y * L.lo;
+  const double nd = floor(Eh * HG_POW_INV_LN2_256 + 0.5);
+  const int n = (int)nd, j = n & 255, q = (n - j) / 256;
+  const hg_dd nc = hg_dd_prod(nd, HG_POW_C2);
+  const hg_dd R = hg_dd_two_sum(Eh - nd * HG_POW_C1, -nc.hi); /* the product is exact, and the difference */
+  const double rh = R.hi, rl = R.lo + ((El - nc.lo) - nd * HG_POW_C3);
+  const double r2 = rh * rh;
+  const double A = r2 * ((0.5 + rh * HG_POW_SIXTH_HI) + r2 * (HG_POW_INV24 + rh * HG_POW_INV120 + r2 * HG_POW_INV720));
+  const double pw = A + (rl + rl * (rh + A));
+  const hg_dd T = hg_pow_exp2(j);
+  const hg_dd t = hg_dd_prod(T.hi, rh);
+  const hg_dd s = hg_dd_fast_sum(T.hi, t.hi);
+  const double lo = s.lo + (t.lo + (T.lo + (T.hi * pw + T.lo * rh)));
+  const double eps = 0x1p-65;
+  const double v = s.hi + (lo - eps);
+  *out = v * hg_pow_from_bits((uint64_t)(q + 1023) << 52);
+  return v == s.hi + (lo + eps);
+}
+
 /* x^y rounded to nearest (see the file comment for the domain). */
 HG_PHD double hg_cr_pow(double x, double y)
 {
@@ -210,6 +288,8 @@ HG_PHD double hg_cr_pow(double x, double y)
   if (x == 1.0) return 1.0;
   if (y == -1.0) return 1.0 / x;
   if (y == 0.5) return sqrt(x);
+  double v;
+  if (fabs(y) <= 2.0 && hg_pow_quick(x, y, &v)) return v;
   const hg_dd E = hg_dd_mul_d(hg_dd_log(x), y);
   if (!(fabs(E.hi) < 700.0)) return pow(x, y);
   return hg_dd_exp_rn(E);
