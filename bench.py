@@ -194,16 +194,17 @@ def peak_hbm():
 def algorithmic_bytes(kind, n):
     """Algorithmic HBM bytes of one launch of a kernel class (FP64 state).
 
-    flux (one direction): every zone of the stencil box read once (8 prims)
-    plus the 8 flux components written once per face.  update: p, p_h read,
+    flux (one launch, three directions): every zone of the stencil box read
+    once per direction (8 prims) plus 8 flux components written once per face
+    (known-zero kernels write 7).  update: p, p_h read,
     five non-induction flux components of the three face families, three
     EMFs and two floors read once per zone; p_f (8), p_gamma and pflag
     written once per zone."""
     N0, N1, N2 = n
     T = [x + 6 for x in n]
     if kind == "flux":
-        faces = (N0 + 1) * T[1] * T[2]
-        return 64.0 * T[0] * T[1] * T[2] + 64.0 * faces
+        faces = (N0 + 1) * T[1] * T[2] + T[0] * (N1 + 1) * T[2] + T[0] * T[1] * (N2 + 1)
+        return 3 * 64.0 * T[0] * T[1] * T[2] + 64.0 * faces
     if kind == "update":
         return (64 + 64 + 3 * 40 + 24 + 16 + 64 + 8 + 4) * float(N0 * N1 * N2)
     if kind == "emf":
@@ -427,7 +428,6 @@ def run_ours(args, wl, rank, world, device):
     out["e2e"] = {"value": e2e_val, "unit": "zone-updates/s",
                   "h2d_bytes_per_step": float(state_bytes) / args.steps,
                   "d2h_bytes_per_step": float(state_bytes) / args.steps + 16 + 120}
-    total_launches = sum(v[1] for v in kt.values()) + 2 * args.steps  # k_begin launches are in "misc"
     out["gpu_launches"] = int(sum(v[1] for v in kt.values()))
     out["nfail_per_step"] = nfail_per_step
     if clocks:

@@ -295,8 +295,18 @@ extern "C" int hg_init(const hg_grid_desc *desc, hg_handle **out)
     h->L.grid_upd = grid_for(G.capacity, 128);
     h->L.grid_fix = grid_for(G.capacity, 2);
     h->L.grid_bnd = grid_for(faces - G.capacity, 16);
-    h->L.strip_nf = 2;  // 2-face strips in all three directions (with these
-    h->L.strip_x1 = 1;  // block counts, the torus's fastest)
+    {
+      // Faces per strip.  Long strips repeat less of the reconstruction;
+      // short ones leave more threads.  One face while every face then has a
+      // thread of its own at once (1024 zones in a line: 0.0725 against
+      // 0.0763 ms per step with 2), two while those strips are no more than
+      // two waves (32^3: 0.1007, with 1 0.1086, with 3 0.1028; 256^2: 0.1396,
+      // 0.1393, 0.1468), else three (96x96x64 torus 0.958 against 0.985 with
+      // 2, 192x192x128 5.38 against 5.64).
+      const long wave = 4L * 128 * sms;
+      h->L.strip_nf = 3 * faces <= wave ? 1 : 3 * faces <= 4 * wave ? 2 : 3;
+    }
+    h->L.strip_x1 = 1;
     {  // the fallback tree: every block the device holds at once, no more
        // than the grid's zones need (small grids in a batch launch few)
       const int fb = fma_kernels(G) ? hg_fma::fallback_blocks_per_sm(G.rescale != 0)

@@ -1,7 +1,7 @@
 // hg_kernels.cu -- sm_100a kernels of one HARM3D time step (step_ch.c:50-234).
 //
 // Per substep (predictor with Dt/2, corrector with Dt):
-//   k_flux x3   one kernel per direction: reconstruction of the six-zone
+//   k_flux_strips  every direction in one launch: reconstruction of the six-zone
 //               stencil of each face (reconstruct_fast, recon.c:894-1103)
 //               fused with get_state/primtoflux/vchar_fast and the HLL or LF
 //               flux (numerical_flux, step_ch.c:636-790); the maximum
@@ -321,6 +321,17 @@ __device__ __forceinline__ void fix_flux(const GridDev &G, int i, long o)
   if (i == G.NE[0] + 1 && *fr < 0) *fr = 0.;
 }
 
+// The faces of one direction: lo, n per axis (reference indices), and how
+// often the reference computes each (its copies of a single zone).
+struct FluxRange {
+  int lo[3], n[3];
+  unsigned mult;
+};
+struct FluxRanges {
+  FluxRange d[3];
+  unsigned first[4];  // first block of each direction
+};
+
 // ---------------------------------------------------------------------------
 // k_flux: F[d] on faces [lo, lo+n) (reference indices), one thread per face.
 template <bool RS, int GM, int d>
@@ -356,7 +367,7 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux(const __gri
 }
 
 // ---------------------------------------------------------------------------
-// k_flux_strip: the faces of a strided direction d (x2 or x3) in strips of
+// flux_strips: the faces of a direction d in strips of
 // NF consecutive faces along d, one strip per thread, lanes along x1.  The
 // thread marches along its strip once per variable, so each zone's slope,
 // interface value and PPM edges are computed once per strip instead of once
@@ -427,12 +438,11 @@ __device__ __forceinline__ void strip_recon(const GridDev &G, const double *__re
 }
 
 template <bool RS, int GM, int d, int NF>
-__global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux_strip(const __grid_constant__ GridDev G,
-                                                                   const double *__restrict__ ph, int lo0, int lo1,
-                                                                   int lo2, int n0, int n1, int n2, unsigned int mult,
-                                                                   int slot, int all)
+__device__ __forceinline__ void flux_strips(const GridDev &G, const double *__restrict__ ph, const FluxRange &R, int slot,
+                                            int all, unsigned first, unsigned step, double *sm)
 {
-  extern __shared__ double sm[];  // 16 * NF * HG_BLK doubles: the strip's face states
+  const int lo0 = R.lo[0], lo1 = R.lo[1], lo2 = R.lo[2], n0 = R.n[0], n1 = R.n[1], n2 = R.n[2];
+  const unsigned mult = R.mult;
   const int tx = threadIdx.x;
   // x2, x3: lanes along x1, one strip per thread along d; x1: consecutive
   // lanes take consecutive strips of the same line
@@ -441,7 +451,7 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux_strip(const
   const unsigned total = (unsigned)nseg * (d == 0 ? n1 * n2 : d == 1 ? n0 * n2 : n0 * n1);  // < 2^31 (hg_init)
   const int st = G.st[d];
   double vmax = 0.;
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+  for (unsigned t = first; t < total; t += step) {
     int seg, i0, j0, k0;
     if (d == 0) {
       const unsigned rest = t / (unsigned)nseg;
@@ -482,6 +492,62 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux_strip(const
     }
   }
   block_max_atomic(vmax, &G.sc->maxs[d + 1]);
+}
+
+// The faces of a direction of one zone: both states are the zone's own.
+template <bool RS, int GM, int d>
+__device__ __forceinline__ void flux_single(const GridDev &G, const double *__restrict__ ph, const FluxRange &R, int slot,
+                                            int all, unsigned first, unsigned step)
+{
+  const unsigned total = (unsigned)R.n[0] * R.n[1] * R.n[2];
+  double vmax = 0.;
+  for (unsigned t = first; t < total; t += step) {
+    const unsigned tq = t / (unsigned)R.n[0];
+    const int i = R.lo[0] + (int)(t - tq * (unsigned)R.n[0]);
+    const int j = R.lo[1] + (int)(tq % (unsigned)R.n[1]);
+    const int k = R.lo[2] + (int)(tq / (unsigned)R.n[1]);
+    const long o = off3(G, i, j, k);
+    double pz[HG_NPR];
+#pragma unroll
+    for (int l = 0; l < HG_NPR; l++) {
+      const double v = __ldg(ph + l * G.S + o);
+      pz[l] = RS ? rs_roundtrip(G, v, l, i) : v;
+    }
+    bool fin;
+    double ctop = flux_at<GM, d>(G, pz, pz, i, j, k, R.mult, o, slot, all, &fin);
+    if (GM >= HG_GM_FLAT && !fin) {
+      double sz[HG_NPR];  // a copy, so that pz stays in registers
+      for (int l = 0; l < HG_NPR; l++) sz[l] = pz[l];
+      ctop = face_flux_full<d>(G, sz, sz, 1, i, j, k, R.mult, o);
+    }
+    if (d == 0 && G.bc == 10) fix_flux(G, i, o);
+    if (i >= HG_NGH && i <= G.NE[0] && j >= HG_NGH && j <= G.NE[1] && k >= HG_NGH && k <= G.NE[2])
+      if (ctop > vmax) vmax = ctop;
+  }
+  block_max_atomic(vmax, &G.sc->maxs[d + 1]);
+}
+
+// Every direction's faces in one launch: blocks [first[d], first[d+1]) take
+// direction d.  The directions do not depend on one another, so a small
+// grid's three launches, each shorter than the device is wide, become one
+// (flux of 1024 zones in a line 57 -> 22 us per step, of 32^3 88 -> 42); a
+// large grid's have one last wave instead of three (96x96x64 torus 0.459 ->
+// 0.421 ms at 2 faces per strip).
+template <bool RS, int GM, int NF>
+__global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux_strips(const __grid_constant__ GridDev G,
+                                                                    const double *__restrict__ ph,
+                                                                    const __grid_constant__ FluxRanges R, int slot, int all)
+{
+  extern __shared__ double sm[];  // 16 * NF * HG_BLK doubles: the strips' face states
+  const int d = blockIdx.x < R.first[1] ? 0 : blockIdx.x < R.first[2] ? 1 : 2;
+  const unsigned t0 = (blockIdx.x - R.first[d]) * HG_BLK + threadIdx.x, step = (R.first[d + 1] - R.first[d]) * HG_BLK;
+#define HG_FLUX_BODY(D)                                                            \
+  if (G.deg[D]) flux_single<RS, GM, D>(G, ph, R.d[D], slot, all, t0, step);         \
+  else flux_strips<RS, GM, D, NF>(G, ph, R.d[D], slot, all, t0, step, sm)
+  if (d == 0) { HG_FLUX_BODY(0); }
+  else if (d == 1) { HG_FLUX_BODY(1); }
+  else { HG_FLUX_BODY(2); }
+#undef HG_FLUX_BODY
 }
 
 // ---------------------------------------------------------------------------
@@ -1596,24 +1662,20 @@ static inline void mark(EventRec *r, int cls, cudaStream_t s)
   r->n++;
 }
 
-// k_flux_strip keeps 16 * NF face states per thread in dynamic shared memory
+// k_flux_strips keeps 16 * NF face states per thread in dynamic shared memory
 // (16, 32 and 48 KiB per block for NF = 1, 2, 3; the limit is raised once
-// per instantiation).  Longer strips save reconstruction work but their
-// shared memory takes L1 capacity from the stencil loads: on the 192^3-class
-// torus NF = 2 measured best, and hg_autotune chooses per grid.
-template <bool RS, int MDIM, int d, int NF>
-static void launch_strip_nf(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, const int *lo,
-                            const int *n, unsigned int mult, int slot, int all)
+// per instantiation).  Longer strips save reconstruction work and leave fewer
+// threads: hg_init chooses by size, hg_autotune on the grid's own state.
+template <bool RS, int MDIM, int NF>
+static void launch_strips_nf(const GridDev &G, cudaStream_t s, const double *ph, const FluxRanges &R, int slot, int all)
 {
-  const size_t smem = sizeof(double) * 16 * NF * HG_BLK;
-  k_flux_strip<RS, MDIM, d, NF>
-      <<<L.grid_flux, HG_BLK, smem, s>>>(G, ph, lo[0], lo[1], lo[2], n[0], n[1], n[2], mult, slot, all);
+  k_flux_strips<RS, MDIM, NF><<<R.first[3], HG_BLK, sizeof(double) * 16 * NF * HG_BLK, s>>>(G, ph, R, slot, all);
 }
 
-template <bool RS, int MDIM, int d, int NF>
+template <bool RS, int MDIM, int NF>
 static cudaError_t strip_attr()
 {
-  return cudaFuncSetAttribute(k_flux_strip<RS, MDIM, d, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(k_flux_strips<RS, MDIM, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(sizeof(double) * 16 * NF * HG_BLK));
 }
 
@@ -1621,9 +1683,7 @@ template <bool RS, int MDIM>
 static cudaError_t strip_attrs_rm()
 {
   cudaError_t e = cudaSuccess;
-  const cudaError_t r[9] = {strip_attr<RS, MDIM, 0, 1>(), strip_attr<RS, MDIM, 0, 2>(), strip_attr<RS, MDIM, 0, 3>(),
-                            strip_attr<RS, MDIM, 1, 1>(), strip_attr<RS, MDIM, 1, 2>(), strip_attr<RS, MDIM, 1, 3>(),
-                            strip_attr<RS, MDIM, 2, 1>(), strip_attr<RS, MDIM, 2, 2>(), strip_attr<RS, MDIM, 2, 3>()};
+  const cudaError_t r[3] = {strip_attr<RS, MDIM, 1>(), strip_attr<RS, MDIM, 2>(), strip_attr<RS, MDIM, 3>()};
   for (cudaError_t x : r)
     if (x != cudaSuccess) e = x;
   return e;
@@ -1658,69 +1718,96 @@ cudaError_t prepare_kernels()
 }
 
 // strips of L.strip_nf faces (1, 2 or 3: a launch-configuration choice)
-template <bool RS, int MDIM, int d>
-static void launch_strip(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, const int *lo,
-                         const int *n, unsigned int mult, int slot, int all)
+template <bool RS, int MDIM>
+static void launch_strips(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, const FluxRanges &R,
+                          int slot, int all)
 {
-  if (L.strip_nf <= 1) launch_strip_nf<RS, MDIM, d, 1>(G, L, s, ph, lo, n, mult, slot, all);
-  else if (L.strip_nf == 2) launch_strip_nf<RS, MDIM, d, 2>(G, L, s, ph, lo, n, mult, slot, all);
-  else launch_strip_nf<RS, MDIM, d, 3>(G, L, s, ph, lo, n, mult, slot, all);
+  if (L.strip_nf <= 1) launch_strips_nf<RS, MDIM, 1>(G, s, ph, R, slot, all);
+  else if (L.strip_nf == 2) launch_strips_nf<RS, MDIM, 2>(G, s, ph, R, slot, all);
+  else launch_strips_nf<RS, MDIM, 3>(G, s, ph, R, slot, all);
 }
 
-static void launch_flux_dir(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, int d,
-                            EventRec *R, int slot, int all)
+// numerical_flux()'s face ranges of direction d
+static FluxRange flux_range(const GridDev &G, int d)
 {
-    int lo[3], n[3];
-    unsigned int mult = 1;
-    for (int a = 0; a < 3; a++) {
-      if (G.deg[a]) {
-        lo[a] = HG_NGH;
-        n[a] = 1;
-        mult *= (a == d) ? 2u : (G.ct_para ? 1u + 2u * HG_NGH : 3u);
-      } else if (a == d) {
-        lo[a] = HG_NGH;
-        n[a] = G.N[a] + 1;
-      } else if (G.ct_para) {
-        lo[a] = 0;
-        n[a] = G.N[a] + 2 * HG_NGH;
-      } else {
-        lo[a] = HG_NGH - 1;
-        n[a] = G.N[a] + 2;
-      }
-    }
-    mark(R, KC_FLUX, s);
-    if (G.prec == HG_PREC_MIXED) {
-      launch_flux_f32(G, L, s, d, lo, n, mult, slot, all);  // reads G.p32, filled from ph
-      return;
-    }
-#define HG_FLUX(RSV, MD, DD) \
-  k_flux<RSV, MD, DD><<<L.grid_flux, HG_BLK, 0, s>>>(G, ph, lo[0], lo[1], lo[2], n[0], n[1], n[2], mult, slot, \
-                                                all)
-#define HG_STRIP(RSV, MD, DD) \
-  launch_strip<RSV, MD, DD>(G, L, s, ph, lo, n, mult, slot, all)
-#define HG_FLUX_D(RSV, MD) \
-  if (d == 0) { if (G.deg[0] || !L.strip_x1) HG_FLUX(RSV, MD, 0); else HG_STRIP(RSV, MD, 0); } \
-  else if (d == 1) { if (G.deg[1]) HG_FLUX(RSV, MD, 1); else HG_STRIP(RSV, MD, 1); } \
-  else { if (G.deg[2]) HG_FLUX(RSV, MD, 2); else HG_STRIP(RSV, MD, 2); }
-    // hg_face_flux (all) takes every entry of the geometry, so that the
-    // signs of its zeros are the reference's too
-    const int gk = all ? HG_GK_FULL : G.gk;
-    if (G.mdim == 0) {
-      if (G.rescale) { HG_FLUX_D(true, HG_GM_CONST) }
-      else if (gk == HG_GK_FLAT) { HG_FLUX_D(false, HG_GM_FLAT) }
-      else { HG_FLUX_D(false, HG_GM_CONST) }
-    } else if (G.mdim == 3) {  // geometry of time level `slot`
-      if (G.rescale) { HG_FLUX_D(true, HG_GM_DYN) }
-      else { HG_FLUX_D(false, HG_GM_DYN) }
-    } else if (gk == HG_GK_AXI) {
-      if (G.rescale) { HG_FLUX_D(true, HG_GM_AXI) }
-      else { HG_FLUX_D(false, HG_GM_AXI) }
+  FluxRange r;
+  r.mult = 1;
+  for (int a = 0; a < 3; a++) {
+    if (G.deg[a]) {
+      r.lo[a] = HG_NGH;
+      r.n[a] = 1;
+      r.mult *= (a == d) ? 2u : (G.ct_para ? 1u + 2u * HG_NGH : 3u);
+    } else if (a == d) {
+      r.lo[a] = HG_NGH;
+      r.n[a] = G.N[a] + 1;
+    } else if (G.ct_para) {
+      r.lo[a] = 0;
+      r.n[a] = G.N[a] + 2 * HG_NGH;
     } else {
-      if (G.rescale) { HG_FLUX_D(true, HG_GM_TAB) }
-      else { HG_FLUX_D(false, HG_GM_TAB) }
+      r.lo[a] = HG_NGH - 1;
+      r.n[a] = G.N[a] + 2;
     }
-#undef HG_FLUX_D
-#undef HG_STRIP
+  }
+  return r;
+}
+
+// Fluxes of the directions d0 .. d1 (hg_face_flux: one of them, all = 1).
+static void launch_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ph, int d0, int d1, EventRec *Rec,
+                        int slot, int all)
+{
+  if (G.prec == HG_PREC_MIXED) {
+    for (int d = d0; d <= d1; d++) {
+      const FluxRange r = flux_range(G, d);
+      mark(Rec, KC_FLUX, s);
+      launch_flux_f32(G, L, s, d, r.lo, r.n, r.mult, slot, all);  // reads G.p32, filled from ph
+    }
+    return;
+  }
+  FluxRanges R;
+  bool per_face = false;
+  unsigned blocks = 0;
+  for (int d = 0; d < 3; d++) {
+    R.d[d] = flux_range(G, d);
+    R.first[d] = blocks;
+    if (d < d0 || d > d1) continue;
+    if (d == 0 && !G.deg[0] && !L.strip_x1) {
+      per_face = true;
+      continue;
+    }
+    const FluxRange &r = R.d[d];
+    long work = (long)r.n[0] * r.n[1] * r.n[2];
+    if (!G.deg[d]) work = work / r.n[d] * ((r.n[d] + L.strip_nf - 1) / L.strip_nf);
+    const long b = (work + HG_BLK - 1) / HG_BLK;
+    blocks += (unsigned)(b < L.grid_flux ? b : L.grid_flux);
+  }
+  R.first[3] = blocks;
+  mark(Rec, KC_FLUX, s);
+  // x1 faces one per thread (a launch-configuration choice)
+#define HG_FLUX(RSV, MD)                                                                                              \
+  {                                                                                                                   \
+    const FluxRange &r = R.d[0];                                                                                      \
+    if (per_face)                                                                                                     \
+      k_flux<RSV, MD, 0><<<L.grid_flux, HG_BLK, 0, s>>>(G, ph, r.lo[0], r.lo[1], r.lo[2], r.n[0], r.n[1], r.n[2],     \
+                                                        r.mult, slot, all);                                           \
+    if (blocks) launch_strips<RSV, MD>(G, L, s, ph, R, slot, all);                                                    \
+  }
+  // hg_face_flux (all) takes every entry of the geometry, so that the
+  // signs of its zeros are the reference's too
+  const int gk = all ? HG_GK_FULL : G.gk;
+  if (G.mdim == 0) {
+    if (G.rescale) HG_FLUX(true, HG_GM_CONST)
+    else if (gk == HG_GK_FLAT) HG_FLUX(false, HG_GM_FLAT)
+    else HG_FLUX(false, HG_GM_CONST)
+  } else if (G.mdim == 3) {  // geometry of time level `slot`
+    if (G.rescale) HG_FLUX(true, HG_GM_DYN)
+    else HG_FLUX(false, HG_GM_DYN)
+  } else if (gk == HG_GK_AXI) {
+    if (G.rescale) HG_FLUX(true, HG_GM_AXI)
+    else HG_FLUX(false, HG_GM_AXI)
+  } else {
+    if (G.rescale) HG_FLUX(true, HG_GM_TAB)
+    else HG_FLUX(false, HG_GM_TAB)
+  }
 #undef HG_FLUX
 }
 
@@ -1736,7 +1823,7 @@ static void launch_substep(const GridDev &G, const LaunchCfg &L, cudaStream_t s,
     k_conn_dyn<<<L.grid_upd, HG_BLK, 0, s>>>(G, sub, 0.5 * sub);
   }
   // (the mixed form's FP32 copy of ph is already current: put_state)
-  for (int d = 0; d < 3; d++) launch_flux_dir(G, L, s, ph, d, R, sub, 0);
+  launch_flux(G, L, s, ph, 0, 2, R, sub, 0);
   {
     int lo[3], n[3];
     for (int a = 0; a < 3; a++) {
@@ -1916,7 +2003,7 @@ void launch_face_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int 
 {
   k_reset_max<<<1, 1, 0, s>>>(G.sc, d + 1);
   if (G.prec == HG_PREC_MIXED) launch_to_f32(G, L.grid_upd, s, G.p);
-  launch_flux_dir(G, L, s, G.p, d, nullptr, 0, 1);
+  launch_flux(G, L, s, G.p, d, d, nullptr, 0, 1);
 }
 
 void launch_fixup_bounds(const GridDev &G, const LaunchCfg &L, cudaStream_t s)
