@@ -302,7 +302,7 @@ extern "C" int hg_init(const hg_grid_desc *desc, hg_handle **out)
       // 0.0763 ms per step with 2), two while those strips are no more than
       // two waves (32^3: 0.1007, with 1 0.1086, with 3 0.1028; 256^2: 0.1396,
       // 0.1393, 0.1468), else three (96x96x64 torus 0.958 against 0.985 with
-      // 2, 192x192x128 5.38 against 5.64).
+      // 2, 192x192x128 5.43 against 5.67, its mixed form 4.02 against 4.19).
       const long wave = 4L * 128 * sms;
       h->L.strip_nf = 3 * faces <= wave ? 1 : 3 * faces <= 4 * wave ? 2 : 3;
     }
