@@ -185,11 +185,47 @@ __device__ __forceinline__ void face_geom_f32(const GridDev &G, int i, int j, Ge
   g.g = __ldg(t + 27 * s);
 }
 
+// Known zeros in FP32.  A component above 3.4e38 is infinite here, and a sum
+// that holds 0 * inf is NaN.  The FP64 kernels take such faces again with
+// every entry; here that call's registers would cost the flux of a 128^3 flat
+// step 0.553 -> 0.581 ms, so the zeros that decide stay, one multiply-add
+// each (0.553 -> 0.554 ms; of a 192x192x128 torus step 1.428 -> 1.440): in
+// u^i = pr - u^0 beta^i, so that an infinite u^0 makes u^i and through it b^a
+// NaN, and for the tables in gamma's quadratic form and in two of the lowered
+// components, so that an infinite b^a makes b^2 NaN (in flat space it is: b^0
+// is infinite too, and b^2 holds -inf + inf).  From b^2 eta and so every
+// stress is NaN, as with every entry.
+__device__ __forceinline__ float quad3(const GeomAxiT<float> &g, float a, float b, float c)
+{
+  return quad3_axi(g, a, b, c) + 0.f * a + 0.f * b + 0.f * c;
+}
+__device__ __forceinline__ void ucon_of(const float *pr, float gamma, const GeomFlatT<float> &, float *ucon)
+{
+  ucon[0] = gamma;
+  ucon[1] = pr[U1] - gamma * 0.f;
+  ucon[2] = pr[U2] - gamma * 0.f;
+  ucon[3] = pr[U3] - gamma * 0.f;
+}
+__device__ __forceinline__ void ucon_of(const float *pr, float gamma, const GeomAxiT<float> &g, float *ucon)
+{
+  ucon[0] = gamma * g.nc0;
+  ucon[1] = pr[U1] - ucon[0] * g.b0;
+  ucon[2] = pr[U2] - ucon[0] * 0.f;
+  ucon[3] = pr[U3] - ucon[0] * 0.f;
+}
+__device__ __forceinline__ void lower4(const float *v, const GeomAxiT<float> &g, float *w)
+{
+  w[0] = g.c00 * v[0] + g.c01 * v[1] + g.c03 * v[3] + 0.f * v[2];
+  w[1] = g.c01 * v[0] + g.c11 * v[1] + g.c13 * v[3];
+  w[2] = g.c22 * v[2] + 0.f * v[1] + 0.f * v[3];
+  w[3] = g.c03 * v[0] + g.c13 * v[1] + g.c33 * v[3];
+}
+
 // HLL/LF flux of one face from FP32 states; returns ctop.  Without the
 // products with a geometry's known zeros (issue-bound kernels): flux of a
 // 128^3 flat step 0.762 -> 0.643 ms, of a 192x192x128 torus step 1.73 -> 1.61.
-// The normal field
-// component, which flux-CT replaces, is left out unless `all` is set.
+// The normal field component, which flux-CT replaces, is left out unless
+// `all` is set.
 template <int d, class GT>
 __device__ __forceinline__ float face_flux_f32(const GridDev &G, const GT &g, const float *pl, const float *pr, int i,
                                                int j, int k, unsigned int mult, long o, int all)

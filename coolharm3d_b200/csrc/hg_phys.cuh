@@ -183,7 +183,8 @@ struct FastDiv {
 // can differ), so face_flux and cons_zone check that the states are finite
 // and the sums that consume their results (update_zone, k_emf) start from or
 // add +0, which takes the sign back; k_update_c2p checks its conserved
-// variables.
+// variables.  The FP32 kernels keep the zeros that decide where a component is
+// infinite instead of checking (hg_mixed.cu).
 template <class T>
 struct GeomFlatT {
   __device__ T ginv() const { return T(1); }
