@@ -30,7 +30,7 @@ void launch_mirror_check(const GridDev &G, int grid, cudaStream_t s, const doubl
 void launch_face_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int d);
 void launch_fixup_bounds(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
 void launch_bounds_only(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
-cudaError_t prepare_kernels();
+cudaError_t prepare_kernels(const GridDev &G);
 int fallback_blocks_per_sm(bool rs);
 void launch_geom_levels(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
 void launch_conn_broadcast(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *rows);
@@ -47,7 +47,7 @@ namespace hg_fma {
 void launch_step(const hg::GridDev &G, const hg::LaunchCfg &L, cudaStream_t s, hg::EventRec *R);
 void launch_geom_levels(const hg::GridDev &G, const hg::LaunchCfg &L, cudaStream_t s);
 void launch_face_flux(const hg::GridDev &G, const hg::LaunchCfg &L, cudaStream_t s, int d);
-cudaError_t prepare_kernels();
+cudaError_t prepare_kernels(const hg::GridDev &G);
 int fallback_blocks_per_sm(bool rs);
 }  // namespace hg_fma
 
@@ -235,7 +235,7 @@ extern "C" int hg_init(const hg_grid_desc *desc, hg_handle **out)
     if ((rc = dev_alloc(h, &q_, (bytes))) != HG_OK) goto fail; \
     ptr = (decltype(ptr))q_;                                  \
   } while (0)
-  if (hg::prepare_kernels() != cudaSuccess || hg_fma::prepare_kernels() != cudaSuccess ||
+  if ((fma_kernels(G) ? hg_fma::prepare_kernels(G) : hg::prepare_kernels(G)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     delete h;

@@ -1666,8 +1666,8 @@ static inline void mark(EventRec *r, int cls, cudaStream_t s)
 }
 
 // k_flux_strips keeps 16 * NF face states per thread in dynamic shared memory
-// (16, 32 and 48 KiB per block for NF = 1, 2, 3; the limit is raised once
-// per instantiation).  Longer strips save reconstruction work and leave fewer
+// (16, 32 and 48 KiB per block for NF = 1, 2, 3; for 3 prepare_kernels raises
+// the limit).  Longer strips save reconstruction work and leave fewer
 // threads: hg_init chooses by size, hg_autotune on the grid's own state.
 template <bool RS, int MDIM, int NF>
 static void launch_strips_nf(const GridDev &G, cudaStream_t s, const double *ph, const FluxRanges &R, int slot, int all)
@@ -1675,21 +1675,11 @@ static void launch_strips_nf(const GridDev &G, cudaStream_t s, const double *ph,
   k_flux_strips<RS, MDIM, NF><<<R.first[3], HG_BLK, sizeof(double) * 16 * NF * HG_BLK, s>>>(G, ph, R, slot, all);
 }
 
-template <bool RS, int MDIM, int NF>
+template <bool RS, int MDIM>
 static cudaError_t strip_attr()
 {
-  return cudaFuncSetAttribute(k_flux_strips<RS, MDIM, NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(sizeof(double) * 16 * NF * HG_BLK));
-}
-
-template <bool RS, int MDIM>
-static cudaError_t strip_attrs_rm()
-{
-  cudaError_t e = cudaSuccess;
-  const cudaError_t r[3] = {strip_attr<RS, MDIM, 1>(), strip_attr<RS, MDIM, 2>(), strip_attr<RS, MDIM, 3>()};
-  for (cudaError_t x : r)
-    if (x != cudaSuccess) e = x;
-  return e;
+  return cudaFuncSetAttribute(k_flux_strips<RS, MDIM, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(sizeof(double) * 16 * 3 * HG_BLK));
 }
 
 // Blocks of k_fallback one SM holds at once.  Each queued zone is one long
@@ -1705,19 +1695,26 @@ int fallback_blocks_per_sm(bool rs)
   return (e == cudaSuccess && n > 0) ? n : 2;
 }
 
-// Kernel attributes that must be set before a launch (the strip kernels'
-// shared memory above the default limit), once per device, outside any
-// stream capture: called by hg_init.
-cudaError_t prepare_kernels()
+// Kernel attributes that must be set before a launch, outside any stream
+// capture: called by hg_init for the build the grid's steps run.  Only 3-face
+// strips pass the default limit (48 KiB, their block reduction's words
+// included).  Setting an attribute loads its kernel and its build's module, so
+// only the one or two that this grid can launch are touched: the first
+// hg_init of a process 93 -> 59 ms (every kernel of both builds before).
+cudaError_t prepare_kernels(const GridDev &G)
 {
-  const cudaError_t r[9] = {strip_attrs_rm<false, HG_GM_CONST>(), strip_attrs_rm<true, HG_GM_CONST>(),
-                            strip_attrs_rm<false, HG_GM_TAB>(),   strip_attrs_rm<true, HG_GM_TAB>(),
-                            strip_attrs_rm<false, HG_GM_DYN>(),   strip_attrs_rm<true, HG_GM_DYN>(),
-                            strip_attrs_rm<false, HG_GM_FLAT>(),  strip_attrs_rm<false, HG_GM_AXI>(),
-                            strip_attrs_rm<true, HG_GM_AXI>()};
-  for (cudaError_t x : r)
-    if (x != cudaSuccess) return x;
-  return cudaSuccess;
+  const bool rs = G.rescale != 0;
+  if (G.prec == HG_PREC_MIXED) return cudaSuccess;  // its fluxes are hg_mixed.cu's
+  if (G.mdim == 3) return rs ? strip_attr<true, HG_GM_DYN>() : strip_attr<false, HG_GM_DYN>();
+  cudaError_t e, k;  // every entry, and its known zeros (hg_set_geometry decides)
+  if (G.mdim == 2) {
+    e = rs ? strip_attr<true, HG_GM_TAB>() : strip_attr<false, HG_GM_TAB>();
+    k = rs ? strip_attr<true, HG_GM_AXI>() : strip_attr<false, HG_GM_AXI>();
+  } else {
+    e = rs ? strip_attr<true, HG_GM_CONST>() : strip_attr<false, HG_GM_CONST>();
+    k = rs ? cudaSuccess : strip_attr<false, HG_GM_FLAT>();
+  }
+  return e != cudaSuccess ? e : k;
 }
 
 // strips of L.strip_nf faces (1, 2 or 3: a launch-configuration choice)
