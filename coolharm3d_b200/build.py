@@ -5,7 +5,9 @@ nvcc flags: -gencode arch=compute_100a,code=sm_100a, -O3, -lineinfo, and
 exactly as in the reference's gcc build and results agree bit for bit.
 The step kernels (hg_kernels.cu) are compiled a second time with
 -fmad=true -DHG_FMA_BUILD into namespace hg_fma: the HG_PREC_FP64_FMA form,
-FP64 with fused multiply-adds (fewer instructions, not bit-identical).
+FP64 with fused multiply-adds (fewer instructions, not bit-identical).  A
+third time, with -DHG_CALLS_BUILD into namespace hg_calls, it gives the kernels
+of the calls outside the step, a small module that every form loads.
 The FP32 kernels of the mixed-precision form (hg_mixed.cu) are not held to
 bit parity: they are built with fused multiply-adds, approximate FP32
 division and square root and flush-to-zero (FP32_FLAGS), which measured
@@ -21,8 +23,10 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libharmgpu.so")
 SOURCES = ["hg_kernels.cu", "hg_api.cu", "hg_geometry.cu", "hg_mixed.cu", "hg_peak.cu"]
 # (object name, source, extra flags): the step kernels once more with fused
-# multiply-adds, into namespace hg_fma (HG_PREC_FP64_FMA)
-EXTRA_OBJECTS = [("hg_kernels_fma.o", "hg_kernels.cu", ["-fmad=true", "-DHG_FMA_BUILD"])]
+# multiply-adds, into namespace hg_fma (HG_PREC_FP64_FMA), and the kernels of
+# the calls outside the step, into namespace hg_calls
+EXTRA_OBJECTS = [("hg_kernels_fma.o", "hg_kernels.cu", ["-fmad=true", "-DHG_FMA_BUILD"]),
+                 ("hg_kernels_calls.o", "hg_kernels.cu", ["-DHG_CALLS_BUILD"])]
 # FP32 kernels of the mixed-precision form may contract multiply-adds
 FMA_SOURCES = {"hg_mixed.cu"}
 FP32_FLAGS = ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"]

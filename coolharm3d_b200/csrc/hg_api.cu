@@ -24,22 +24,28 @@
 
 namespace hg {
 void launch_step(const GridDev &G, const LaunchCfg &L, cudaStream_t s, EventRec *R);
-void *gather_times_kernel();
 void launch_to_f32(const GridDev &G, int grid, cudaStream_t s, const double *src);
 void launch_mirror_check(const GridDev &G, int grid, cudaStream_t s, const double *src, unsigned long long *count);
 void launch_face_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int d);
-void launch_fixup_bounds(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
-void launch_bounds_only(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
 cudaError_t prepare_kernels(const GridDev &G);
 int fallback_blocks_per_sm(bool rs);
 void launch_geom_levels(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
+}  // namespace hg
+
+// What the other calls launch, of every form (hg_kernels.cu compiled with
+// HG_CALLS_BUILD).
+namespace hg_calls {
+using namespace hg;
+void *gather_times_kernel();
+void launch_fixup_bounds(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
+void launch_bounds_only(const GridDev &G, const LaunchCfg &L, cudaStream_t s);
 void launch_conn_broadcast(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *rows);
 void launch_totals(const GridDev &G, const LaunchCfg &L, cudaStream_t s, double *part, double *out);
 void launch_ref_to_planes(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *ref, int NT1, int NT2,
                           double *out);
 void launch_planes_to_ref(const GridDev &G, const LaunchCfg &L, cudaStream_t s, const double *in, int NT0, int NT1,
                           int NT2, double *ref);
-}  // namespace hg
+}  // namespace hg_calls
 
 // The same step kernels built with contracted multiply-adds
 // (hg_kernels.cu compiled with HG_FMA_BUILD): HG_PREC_FP64_FMA.
@@ -650,7 +656,7 @@ static int upload_impl(hg_handle *h, FILL fill, const double *direct = nullptr)
     }
     return e;
   }));
-  hg::launch_ref_to_planes(G, h->L, h->stream, dref, h->NT[1], h->NT[2], G.p);
+  hg_calls::launch_ref_to_planes(G, h->L, h->stream, dref, h->NT[1], h->NT[2], G.p);
   HG_CK(cudaGetLastError());
   HG_CK(cudaMemsetAsync(G.nfail, 0, sizeof(unsigned int) * HG_NF * G.S, h->stream));
   HG_CK(cudaMemsetAsync(G.pflag, 0, sizeof(int) * G.S, h->stream));
@@ -669,7 +675,7 @@ static int download_impl(hg_handle *h, DRAIN drain, double *direct = nullptr)
   HG_CK(cudaSetDevice(h->d.device));
   double *dref = ref_buffer(h);
   if (!dref) return HG_ERR_NOMEM;
-  hg::launch_planes_to_ref(G, h->L, h->stream, G.p, h->NT[0], h->NT[1], h->NT[2], dref);
+  hg_calls::launch_planes_to_ref(G, h->L, h->stream, G.p, h->NT[0], h->NT[1], h->NT[2], dref);
   HG_CK(cudaGetLastError());
   if (direct) {
     HG_CK(cudaMemcpyAsync(direct, dref, sizeof(double) * HG_NPR * h->ntot_ref, cudaMemcpyDeviceToHost, h->stream));
@@ -915,7 +921,7 @@ extern "C" int hg_set_dynamic_metric(hg_handle *h, const hg_dyn_metric *m)
     cudaError_t e = cudaMemcpyAsync(drows, rows.data(), sizeof(double) * rows.size(), cudaMemcpyHostToDevice,
                                     h->stream);
     if (e == cudaSuccess) {
-      hg::launch_conn_broadcast(h->G, h->L, h->stream, (const double *)drows);
+      hg_calls::launch_conn_broadcast(h->G, h->L, h->stream, (const double *)drows);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -1049,7 +1055,7 @@ extern "C" int hg_fixup_bounds(hg_handle *h)
   HG_CK(cudaSetDevice(h->d.device));
   int rc = refresh_levels(h);
   if (rc != HG_OK) return rc;
-  hg::launch_fixup_bounds(h->G, h->L, h->stream);
+  hg_calls::launch_fixup_bounds(h->G, h->L, h->stream);
   HG_CK(cudaGetLastError());
   HG_CK(cudaStreamSynchronize(h->stream));
   return HG_OK;
@@ -1300,7 +1306,7 @@ static int batch_rebuild(hg_batch *b)
     double *out = b->d_out;
     void *args[] = {&scp, &nn, &out};
     cudaKernelNodeParams kp = {};
-    kp.func = hg::gather_times_kernel();
+    kp.func = hg_calls::gather_times_kernel();
     kp.gridDim = dim3(1);
     kp.blockDim = dim3(128);
     kp.kernelParams = args;
@@ -1495,7 +1501,7 @@ extern "C" int hg_get_totals(hg_handle *h, double U_tot[8], double F_tot[48], do
     int rc = refresh_levels(h);
     if (rc != HG_OK) return rc;
   }
-  hg::launch_totals(h->G, h->L, h->stream, h->d_tot, out);
+  hg_calls::launch_totals(h->G, h->L, h->stream, h->d_tot, out);
   HG_CK(cudaGetLastError());
   double v[57];
   HG_CK(copy_sync(h, v, out, sizeof(v), cudaMemcpyDeviceToHost));
@@ -1850,7 +1856,7 @@ extern "C" int hg_read_rdump(hg_handle *h, const char *path, int32_t *nstep, int
     h->G.grid_length[0] = gl0;
     h->d.grid_length[0] = gl0;
     h->graph_dirty = true;
-    hg::launch_bounds_only(h->G, h->L, h->stream);
+    hg_calls::launch_bounds_only(h->G, h->L, h->stream);
     HG_CK(cudaGetLastError());
     HG_CK(cudaStreamSynchronize(h->stream));
   }

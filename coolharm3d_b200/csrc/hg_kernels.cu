@@ -30,14 +30,21 @@
 #include "hg_dyn.cuh"
 #include "hg_fallback.cuh"
 
-// This file is compiled twice.  Plain: into namespace hg with no multiply-add
-// contracted (-fmad=false), every FP64 operation rounded as in the
-// reference's build (HG_PREC_FP64, bit-identical results).  With HG_FMA_BUILD
-// and -fmad=true: the same kernels and launch sequence into namespace hg_fma,
-// where the compiler fuses multiply-adds (HG_PREC_FP64_FMA: fewer FP64
-// instructions, results within rounding of the plain form).  Types and the
-// device functions of the headers are shared through namespace hg.
-#ifdef HG_FMA_BUILD
+// This file is compiled three times.  Plain: the step into namespace hg with
+// no multiply-add contracted (-fmad=false), every FP64 operation rounded as in
+// the reference's build (HG_PREC_FP64, bit-identical results).  With
+// HG_FMA_BUILD and -fmad=true: the same kernels and launch sequence into
+// namespace hg_fma, where the compiler fuses multiply-adds (HG_PREC_FP64_FMA:
+// fewer FP64 instructions, results within rounding of the plain form).  With
+// HG_CALLS_BUILD and -fmad=false: what every form's other calls launch
+// (transfers, set-up fixups, totals) into namespace hg_calls, a small module
+// of its own, because the first launch of a kernel loads its module: mixed and
+// FMA grids never load the plain step's (first upload and fixup of a process
+// with a 1024-zone grid: FMA 31 -> 2 ms, mixed 46 -> 16).  Types and the device
+// functions of the headers are shared through namespace hg.
+#if defined(HG_CALLS_BUILD)
+#define HG_KNS hg_calls
+#elif defined(HG_FMA_BUILD)
 #define HG_KNS hg_fma
 #else
 #define HG_KNS hg
@@ -1390,6 +1397,7 @@ __global__ void __launch_bounds__(HG_BLK) k_fixup(GridDev G, double *__restrict_
   }
 }
 
+#ifdef HG_CALLS_BUILD
 // ---------------------------------------------------------------------------
 // fixup(), fixup.c:8-33 with fixup1zone (fixup.c:45-75): over the physical
 // zones, gamma_calc (FAIL_GAMMA_CALC, gamma = 1 on failure), the rho/u floors
@@ -1444,6 +1452,7 @@ __global__ void k_begin(DevScalars *sc)
   sc->fl_count = 0;
 }
 
+#else   // the step builds
 // t += dx[0]; dx[0] = timestep() (step_ch.c:218-223, 546-623); M_tot.
 __global__ void k_timestep(GridDev G, int nblk)
 {
@@ -1870,6 +1879,40 @@ static void launch_substep(const GridDev &G, const LaunchCfg &L, cudaStream_t s,
 
 __global__ void k_reset_max(DevScalars *sc, int dim) { sc->maxs[dim] = 0ull; }
 
+// Fluxes of direction d from the resident primitives G.p (hg_face_flux).
+void launch_face_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int d)
+{
+  k_reset_max<<<1, 1, 0, s>>>(G.sc, d + 1);
+  if (G.prec == HG_PREC_MIXED) launch_to_f32(G, L.grid_upd, s, G.p);
+  launch_flux(G, L, s, G.p, d, d, nullptr, 0, 1);
+}
+
+void launch_step(const GridDev &G, const LaunchCfg &L, cudaStream_t s, EventRec *R)
+{
+  launch_substep(G, L, s, 0, R);
+  launch_substep(G, L, s, 1, R);
+  mark(R, KC_MISC, s);
+  k_timestep<<<1, 1024, 0, s>>>(G, L.grid_upd);
+  if (G.mdim == 3) {  // advance_geometry() at the end of step_ch() (step_ch.c:225-227)
+    mark(R, KC_GEOM, s);
+    k_advance_geometry<<<1, 1, 0, s>>>(G.sc);
+    launch_geom_level(G, L, s, 1, 0.5);
+    launch_geom_level(G, L, s, 2, 1.0);
+  }
+  mark(R, KC_END, s);
+}
+
+// all three time levels at t (init_general_metric, metric.c:3664-3690)
+void launch_geom_levels(const GridDev &G, const LaunchCfg &L, cudaStream_t s)
+{
+  launch_geom_level(G, L, s, 0, 0.0);
+  launch_geom_level(G, L, s, 1, 0.5);
+  launch_geom_level(G, L, s, 2, 1.0);
+}
+
+#endif  // HG_CALLS_BUILD
+
+#ifdef HG_CALLS_BUILD
 // ---------------------------------------------------------------------------
 // Layout conversion between the reference's p[i][j][k][l] (NP innermost,
 // every direction N+6 long) and the resident planes.  One thread per stored
@@ -1996,14 +2039,6 @@ void launch_planes_to_ref(const GridDev &G, const LaunchCfg &L, cudaStream_t s, 
                             s>>>(G, in, NT1, NT2, ref);
   else
     k_planes_to_ref<<<L.grid_flux, HG_BLK, 0, s>>>(G, in, NT0, NT1, NT2, ref);
-}
-
-// Fluxes of direction d from the resident primitives G.p (hg_face_flux).
-void launch_face_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, int d)
-{
-  k_reset_max<<<1, 1, 0, s>>>(G.sc, d + 1);
-  if (G.prec == HG_PREC_MIXED) launch_to_f32(G, L.grid_upd, s, G.p);
-  launch_flux(G, L, s, G.p, d, d, nullptr, 0, 1);
 }
 
 void launch_fixup_bounds(const GridDev &G, const LaunchCfg &L, cudaStream_t s)
@@ -2170,21 +2205,6 @@ void launch_bounds_only(const GridDev &G, const LaunchCfg &L, cudaStream_t s)
   if (G.p32) launch_to_f32(G, L.grid_upd, s, G.p);
 }
 
-void launch_step(const GridDev &G, const LaunchCfg &L, cudaStream_t s, EventRec *R)
-{
-  launch_substep(G, L, s, 0, R);
-  launch_substep(G, L, s, 1, R);
-  mark(R, KC_MISC, s);
-  k_timestep<<<1, 1024, 0, s>>>(G, L.grid_upd);
-  if (G.mdim == 3) {  // advance_geometry() at the end of step_ch() (step_ch.c:225-227)
-    mark(R, KC_GEOM, s);
-    k_advance_geometry<<<1, 1, 0, s>>>(G.sc);
-    launch_geom_level(G, L, s, 1, 0.5);
-    launch_geom_level(G, L, s, 2, 1.0);
-  }
-  mark(R, KC_END, s);
-}
-
 // conn3 of the physical zones from rows (j + N1 i) of 64 that do not depend
 // on k (a static axisymmetric connection)
 __global__ void k_conn_broadcast(GridDev G, const double *rows)
@@ -2206,17 +2226,11 @@ void launch_conn_broadcast(const GridDev &G, const LaunchCfg &L, cudaStream_t s,
   k_conn_broadcast<<<L.grid_upd, HG_BLK, 0, s>>>(G, rows);
 }
 
-// all three time levels at t (init_general_metric, metric.c:3664-3690)
-void launch_geom_levels(const GridDev &G, const LaunchCfg &L, cudaStream_t s)
-{
-  launch_geom_level(G, L, s, 0, 0.0);
-  launch_geom_level(G, L, s, 1, 0.5);
-  launch_geom_level(G, L, s, 2, 1.0);
-}
+#endif  // HG_CALLS_BUILD
 
 }  // namespace HG_KNS
 
-#ifndef HG_FMA_BUILD
+#ifdef HG_CALLS_BUILD
 
 // ===========================================================================
 // hg_face_flux_noalloc: hg_face_flux for callers that cannot allocate device
@@ -2230,7 +2244,7 @@ void launch_geom_levels(const GridDev &G, const LaunchCfg &L, cudaStream_t s)
 // (so a cudaDeviceReset, which reloads the module at a new address, is
 // followed), and taken from the last lookup on that device during capture.
 // ===========================================================================
-namespace hg {
+namespace hg_calls {
 
 #define HG_NA_MAX_BLOCKS 32768  // one block per 128 faces: at most 4,194,304 faces per call
 static __device__ __align__(256) unsigned long long hg_na_scratch[HG_NA_MAX_BLOCKS + 32];
@@ -2325,7 +2339,7 @@ __global__ void __launch_bounds__(HG_BLK) k_flux_noalloc(const __grid_constant__
   }
 }
 
-}  // namespace hg
+}  // namespace hg_calls
 
 #include <mutex>
 
@@ -2334,7 +2348,7 @@ __global__ void __launch_bounds__(HG_BLK) k_flux_noalloc(const __grid_constant__
 extern "C" int hg_face_flux_noalloc(const hg_grid_desc *d, const double *geom, const double *prims, double *flux,
                                     double *max_char_speed, int32_t dir, void *stream)
 {
-  using namespace hg;
+  using namespace hg_calls;
   if (!d || !geom || !prims || !flux || !max_char_speed || dir < 0 || dir > 2) return HG_ERR_BADARG;
   if (d->metric_dim != 0 || d->rescale_r != 0 || d->n1 < 2 || d->n2 < 2 || d->n3 < 2) return HG_ERR_BADARG;
   if (d->recon_type < 0 || d->recon_type > 5 || (d->flux_type != 0 && d->flux_type != 1)) return HG_ERR_BADARG;
@@ -2424,4 +2438,4 @@ extern "C" int hg_face_flux_noalloc(const hg_grid_desc *d, const double *geom, c
   return HG_OK;
 }
 
-#endif  // HG_FMA_BUILD
+#endif  // HG_CALLS_BUILD
