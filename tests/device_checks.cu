@@ -1,7 +1,8 @@
 // device_checks.cu -- small calls into the engine's device code that no entry
 // point of the library makes by itself, for tests/test_device_functions.py:
-// the FP32 flux kernels of hg_mixed.cu (hg::launch_flux_f32 of libharmgpu.so)
-// on given states and geometry.  It returns 0 or the CUDA error.
+// the branch-free divisions of hg_phys.cuh on given operands, and the FP32
+// flux kernels of hg_mixed.cu (hg::launch_flux_f32 of libharmgpu.so) on given
+// states and geometry.  Every function returns 0 or the CUDA error.
 #include <cstring>
 #include <vector>
 
@@ -33,6 +34,33 @@ struct Pool {
   void get(T *dst, const T *src, size_t n) { note(cudaMemcpy(dst, src, n * sizeof(T), cudaMemcpyDeviceToHost)); }
   ~Pool() { for (void *p : ptrs) cudaFree(p); }
 };
+
+// out: a/b, 1/b, 1/b by rcp_any, a/b by div_any, within(a, b, tol); ok of each
+__global__ void k_divisions(int n, const double *a, const double *b, double tol, double *out, unsigned char *ok)
+{
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  FastDiv dv[5];
+  out[t] = dv[0].div(a[t], b[t]);
+  out[n + t] = dv[1].rcp(b[t]);
+  out[2 * n + t] = dv[2].rcp_any(b[t]);
+  out[3 * n + t] = dv[3].div_any(a[t], b[t]);
+  out[4 * n + t] = dv[4].within(a[t], b[t], tol);
+  for (int q = 0; q < 5; q++) ok[q * n + t] = dv[q].ok;
+}
+
+extern "C" int check_divisions(int n, const double *a, const double *b, double tol, double *out, unsigned char *ok)
+{
+  Pool m;
+  double *da = m.make(n, a), *db = m.make(n, b), *dout = m.make<double>(5 * (size_t)n, nullptr);
+  unsigned char *dok = m.make<unsigned char>(5 * (size_t)n, nullptr);
+  if (m.err != cudaSuccess) return m.err;
+  k_divisions<<<(n + 127) / 128, 128>>>(n, da, db, tol, dout, dok);
+  m.note(cudaGetLastError());
+  m.get(out, dout, 5 * (size_t)n);
+  m.get(ok, dok, 5 * (size_t)n);
+  return m.err;
+}
 
 // Fluxes of the three directions on a grid of n physical zones (every
 // direction resolved) from FP32 primitives (8 planes, x1 fastest).  geom: one

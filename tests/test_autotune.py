@@ -30,7 +30,7 @@ def test_autotune_keeps_state_and_results(name):
     np.testing.assert_array_equal(p_tuned, ref.download())
     assert t_tuned == t_ref
     # every strip length gives the same step
-    for nf, x1 in ((1, 1), (3, 0), (2, 1)):
+    for nf, x1 in ((1, 1), (3, 0), (2, 1), (3, 1), (2, 0)):
         cfg2 = e.launch_config()
         cfg2.strip_faces = nf
         cfg2.strip_x1 = x1

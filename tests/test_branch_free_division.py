@@ -1,9 +1,10 @@
 """The divisions of the flux and inversion kernels that are rounded correctly
 without a branch, with their way out where the operands are too small, too
-large or of 53 ones: against the oracle, which divides as C does, and (fluxes)
-against the kernels that take every entry of the geometry.  States over many
-orders of magnitude, fields down to subnormal ones and exactly zero; bit for
-bit, as every division is correctly rounded on both sides."""
+large or of 53 ones: against the oracle, which divides as C does.  States over
+many orders of magnitude, fields down to subnormal ones and exactly zero, with
+strips of every length; bit for bit, as every division is correctly rounded on
+both sides.  (The divisions on given operands: tests/test_device_functions.py;
+against the kernels that take every entry: tests/test_known_zeros.py.)"""
 import numpy as np
 import pytest
 
@@ -33,13 +34,19 @@ def wide_state(f, lo, seed):
 def test_wide_states_against_oracle(name, lo):
     f = fixtures.load(name)
     p0 = wide_state(f, lo, -lo)
-    e, cell6 = engine_for(f["n"], f["sw"], f, p0, f["t0"], f["dt0"])
-    t, dt = e.step(2)
-    p, gamma, fails = e.download(), e.gamma(), e.fail_counts()
-    e.close()
-    o = ht.Oracle(f["n"], f["sw"], fixtures.geomd(f, cell6), lib=ht.CR_ORACLE)
-    o.set_state(p0, f["t0"], f["dt0"])
-    o.step(2)
-    s = o.state()
-    assert np.array_equal(p, s["p"], equal_nan=True)
-    assert fails.tolist() == s["nfailtot"].tolist()
+    o = None
+    for faces, x1 in ((1, 1), (2, 1), (3, 1), (3, 0)):
+        e, cell6 = engine_for(f["n"], f["sw"], f, p0, f["t0"], f["dt0"])
+        c = e.launch_config()
+        c.strip_faces, c.strip_x1 = faces, x1
+        e.set_launch_config(c)
+        t, dt = e.step(2)
+        p, gamma, fails = e.download(), e.gamma(), e.fail_counts()
+        e.close()
+        if o is None:
+            o = ht.Oracle(f["n"], f["sw"], fixtures.geomd(f, cell6), lib=ht.CR_ORACLE)
+            o.set_state(p0, f["t0"], f["dt0"])
+            o.step(2)
+            s = o.state()
+        assert np.array_equal(p, s["p"], equal_nan=True), (faces, x1)
+        assert fails.tolist() == s["nfailtot"].tolist()
