@@ -309,6 +309,12 @@ extern "C" int hg_init(const hg_grid_desc *desc, hg_handle **out)
       // two waves (32^3: 0.1007, with 1 0.1086, with 3 0.1028; 256^2: 0.1396,
       // 0.1393, 0.1468), else three (96x96x64 torus 0.958 against 0.985 with
       // 2, 192x192x128 5.43 against 5.67, its mixed form 4.02 against 4.19).
+      // The wave is that of the FP64 known-zero kernels (4 blocks per SM).
+      // The others (3 blocks; FP32: 7) would draw the line elsewhere: over 99
+      // pairs of grid (128 zones in a line to 96^3) and form (FP64, FMA,
+      // mixed; known zeros, every entry, time-dependent) the choice was within
+      // 6% of the best length, within 1% in 81 of them, and nowhere slower
+      // than strips of 2 in three launches.  hg_autotune measures.
       const long wave = 4L * 128 * sms;
       h->L.strip_nf = 3 * faces <= wave ? 1 : 3 * faces <= 4 * wave ? 2 : 3;
     }

@@ -27,9 +27,9 @@
  * in double; the tables log(1 + k/256) and 2^(j/256) are double-double
  * values computed with 80-digit decimal arithmetic (gen_pow_tables.py).
  * Before that a quick phase of a fifth of the length (hg_pow_quick) computes
- * x^y to within 2^-68 in single steps of double arithmetic with one low word,
- * and returns its rounding where no number that close rounds otherwise (all
- * but one call in 3000).
+ * x^y to within 2^-69 in single steps of double arithmetic with one low word,
+ * and returns its rounding where no number within 2^-65 rounds otherwise (all
+ * but one call in 4100, of 2e7 at random with the entropy fix's exponents).
  * Other inputs (x <= 0, subnormal or infinite x, NaN, |y log x| >= 700) go
  * to the platform's pow(); the step never produces them.
  *

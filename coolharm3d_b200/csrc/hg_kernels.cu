@@ -60,8 +60,9 @@ void launch_to_f32(const GridDev &G, int grid, cudaStream_t s, const double *src
 namespace HG_KNS {
 using namespace hg;
 
-// register caps (minimum resident blocks of 128 threads per SM), measured on
-// the 192x192x128 torus: the flux kernels at 3 blocks (168 registers, no
+// register caps (minimum resident blocks of 128 threads per SM) of the kernels
+// that take every entry of the geometry, measured on the 192x192x128 torus
+// before there were others: the flux kernels at 3 blocks (168 registers, no
 // spills; at 4 blocks, 128 registers, they spilled ~3e6 local-load sectors
 // per launch: 6.36 against 6.70 ms per step); the corrector's conserved
 // update at 3 blocks (168 registers; 4 blocks spill 264 bytes), the
@@ -207,16 +208,16 @@ __device__ __forceinline__ void face_prims(const GridDev &G, const double *__res
 }
 
 // ---------------------------------------------------------------------------
-// HLL/LF flux of a face from its two states; writes the 8 components and
-// returns ctop.  Component by component, so no 32-value temporaries.  The
-// normal field component is left out unless `all` is set: flux-CT replaces
-// it, and only hg_face_flux reads it.  *fin is set to whether the states are
-// finite (known-zero geometries), or to 1.
 __device__ __forceinline__ bool is_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
 __device__ __forceinline__ bool all_ok(const SlowDiv &) { return true; }
 __device__ __forceinline__ bool all_ok(const FastDiv &dv) { return dv.ok; }
 
+// HLL/LF flux of a face from its two states; returns ctop.  Component by
+// component, so no 32-value temporaries.  The normal field component is left
+// out unless `all` is set: flux-CT replaces it, and only hg_face_flux reads
+// it.  *fin is set to whether the states are finite and the branch-free
+// divisions applied (known-zero geometries), or to 1.
 template <int d, class GT>
 __device__ __forceinline__ double face_flux(const GridDev &G, const double *pl, const double *pr, const GT &g,
                                             int i, int j, int k, unsigned int mult, double *__restrict__ Fd, long o,
@@ -343,12 +344,13 @@ struct FluxRanges {
 };
 
 // ---------------------------------------------------------------------------
-// k_flux: F[d] on faces [lo, lo+n) (reference indices), one thread per face.
-template <bool RS, int GM, int d>
+// k_flux: F[0] on faces [lo, lo+n) (reference indices), one thread per face.
+template <bool RS, int GM>
 __global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux(const __grid_constant__ GridDev G, const double *__restrict__ ph,
                                                  int lo0, int lo1, int lo2, int n0, int n1, int n2, unsigned int mult,
                                                  int slot, int all)
 {
+  constexpr int d = 0;
   const unsigned total = (unsigned)n0 * n1 * n2;  // < 2^31 (hg_init)
   double vmax = 0.;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux(const __gri
       }
       ctop = face_flux_full<d>(G, sl, sr, 1, i, j, k, mult, o);
     }
-    if (d == 0 && G.bc == 10) fix_flux(G, i, o);
+    if (G.bc == 10) fix_flux(G, i, o);
     if (i >= HG_NGH && i <= G.NE[0] && j >= HG_NGH && j <= G.NE[1] && k >= HG_NGH && k <= G.NE[2])
       if (ctop > vmax) vmax = ctop;
   }
@@ -385,9 +387,6 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX_BLOCKS(GM)) k_flux(const __gri
 // per zone as well).  The face states wait in shared memory, each thread in
 // its own column, until the strip's fluxes are formed.  Every face value is
 // produced by the same operations on the same inputs as in face_prims.
-#ifndef HG_STRIP_NF
-#define HG_STRIP_NF 2
-#endif
 
 // Face states of NF faces f0 .. f0+NF-1 along d from zones f0-3 .. f0+NF+1
 // of one variable; zones past the strip's nf faces are clamped (their
@@ -1796,7 +1795,7 @@ static void launch_flux(const GridDev &G, const LaunchCfg &L, cudaStream_t s, co
   {                                                                                                                   \
     const FluxRange &r = R.d[0];                                                                                      \
     if (per_face)                                                                                                     \
-      k_flux<RSV, MD, 0><<<L.grid_flux, HG_BLK, 0, s>>>(G, ph, r.lo[0], r.lo[1], r.lo[2], r.n[0], r.n[1], r.n[2],     \
+      k_flux<RSV, MD><<<L.grid_flux, HG_BLK, 0, s>>>(G, ph, r.lo[0], r.lo[1], r.lo[2], r.n[0], r.n[1], r.n[2],     \
                                                         r.mult, slot, all);                                           \
     if (blocks) launch_strips<RSV, MD>(G, L, s, ph, R, slot, all);                                                    \
   }

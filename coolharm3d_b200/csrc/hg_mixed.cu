@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(HG_BLK, HG_FLUX32_MINB) k_flux_f32(const __gri
 }
 
 // Strips of NF consecutive faces along a strided direction (x2, x3), lanes
-// along x1: each zone's PPM edges are formed once per strip (the FP64
-// FP64 strips' scheme); the strip's face states wait in shared memory.
+// along x1: each zone's PPM edges are formed once per strip (the FP64 strips'
+// scheme); the strip's face states wait in shared memory.
 
 // X1 with RESCALE_R: zones scaled by their factors before, face states by
 // their faces' factors after the reconstruction (FP32 copies of the tables).

@@ -648,8 +648,8 @@ __device__ __forceinline__ void ppm_zone(int rt, const T *y, T *ln, T *rn)
 // Con2prim (utoprim_2d_fast.c:135-740).  Returns the reference's codes.
 // Its divisions are dv's, which an iteration overlaps with its square root
 // where they have no branches, and its test |dx/x| <= tol takes none: update
-// of a 128^3 flat step 0.579 -> 0.549 ms, of a 192x192x128 torus step 1.649 ->
-// 1.578.  Plain stay the two whose numerators pass every size where the fluid
+// of a 128^3 flat step 0.553 -> 0.526 ms, of a 192x192x128 torus step 1.571 ->
+// 1.510 (both at 6 blocks per SM).  Plain stay the two whose numerators pass every size where the fluid
 // is at rest or the field ends.
 template <class GT, class DV>
 __device__ __forceinline__ int utoprim_2d(const double *U, const GT &g, double gam, double *prim, double *gamma_out,
